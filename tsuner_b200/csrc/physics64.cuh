@@ -14,6 +14,7 @@
 #include <cfloat>
 #include <cstdint>
 
+#include "ieee64.h"
 #include "tsuner_b200.h"
 
 namespace tsu {
@@ -40,6 +41,11 @@ struct Phys64 {
     // 1: an edge whose two faces are both dry returns zero fluctuations
     // without evaluating the Riemann solver (see edge_flux)
     int dry_skip;
+    double inv_vs;  // RN(1 / k.vs)
+    // High word of a speed s such that two components below it leave the bed
+    // at rest for certain: Opar (s^2 + s^2) < 0.99 OC (0: no such speed).
+    unsigned still_hi;
+    __device__ __forceinline__ bool still(double u) const { return (hi32(u) & 0x7fffffffu) < still_hi; }
 };
 
 // IEEE quotient and square root with the zero cases answered directly:
@@ -126,6 +132,122 @@ struct State5 {
     double h, qx, qy, H, hc;
 };
 
+// What an edge needs of the face on one side: depth, bed, the velocity and
+// the concentration that RiemannSolver_Vols computes from the filtered face
+// (GPU/VolumeSolver.cu:28-36).  They are formed where the face is, because
+// the filter already divides by the same h + EPSILON; the discharge and load
+// themselves are not used by the edge.
+struct Face5 {
+    double h, u, v, H, c;
+};
+
+// Every formula below that divides or takes roots exists in two forms with
+// the same operations in the same order.  FAST: the branch-free quotients and
+// roots of ieee64.h, with `ok` cleared when an operand lies outside the range
+// they are exact in (the results are then not used).  Otherwise: the ordinary
+// operators, any operand.  The range tests read the high words only (integer
+// instructions: the FP64 pipe is the scarcer one).
+template <bool FAST>
+struct Divisor {
+    double d, y;
+    // FAST: mid(d) is the caller's to know
+    __device__ __forceinline__ Divisor(double d_, bool &ok) : d(d_), y(0.0) {
+        if (FAST) {
+            y = recip(d);
+            ok &= recip_ok(d);
+        }
+    }
+    // numerator / d
+    __device__ __forceinline__ double of(double a, bool &ok) const {
+        if (!FAST) return ddiv(a, d);
+        ok &= mid_or_zero(a);
+        return quot(a, d, y);
+    }
+    // FAST: the same without the test
+    __device__ __forceinline__ double of(double a) const { return FAST ? quot(a, d, y) : ddiv(a, d); }
+    // the same for a numerator near q0 * d
+    __device__ __forceinline__ double near(double a, double q0) const {
+        return FAST ? quot_from(a, d, y, q0) : ddiv(a, d);
+    }
+};
+template <bool FAST>
+__device__ __forceinline__ double root_of(double x) {
+    return FAST ? root(x) : dsqrt(x);
+}
+
+// h + EPSILON of a wet state: 2^-19 <= d < 2^100 (d >= 2^-19 implies h > EPS)
+__device__ __forceinline__ bool wet_divisor(double d) { return hi32(d) - 0x3ec00000u < 0x07700000u; }
+// u = q / d of such a state is exact and cannot be clamped together with its
+// other component: q is a zero or 2^-700 <= |u| < 7 (7^2 + 7^2 < VMAX^2)
+__device__ __forceinline__ bool calm(double q, double u) {
+    return ((hi32(u) & 0x7fffffffu) - 0x14300000u < 0x401c0000u - 0x14300000u) |
+           (((hi32(q) & 0x7fffffffu) | lo32(q)) == 0u);
+}
+static_assert(kVmax == 10.0 && kEps < 0x1p-19, "calm, wet_divisor");
+
+// Velocity and concentration of an unfiltered state (a cell, a ghost).
+template <bool FAST>
+__device__ __forceinline__ Face5 face_of(double h, double qx, double qy, double H, double hc, bool &ok) {
+    Face5 f;
+    f.h = h;
+    f.H = H;
+    if (FAST) {
+        const Divisor<true> d(h + kEpsilon, ok);
+        f.u = d.of(qx);
+        f.v = d.of(qy);
+        f.c = d.of(hc, ok);
+        ok &= wet_divisor(d.d) & calm(qx, f.u) & calm(qy, f.v);
+    } else {
+        velocity(h, qx, qy, f.u, f.v);
+        f.c = ddiv(hc, h + kEpsilon);
+    }
+    return f;
+}
+
+// A state through the positivity filter (state_filter_double,
+// GPU/SedFlux.cuh:118-132), and the velocity and concentration of the result;
+// h, qx, qy, hc become the filtered ones.  FAST: a wet, unclamped state (six
+// quotients by the same h + EPSILON) or one without water and load, which
+// comes out as zeros; `dry` says which.
+template <bool FAST>
+__device__ __forceinline__ Face5 filter_face(double &h, double &qx, double &qy, double H, double &hc, bool &ok) {
+    if (!FAST) {
+        positivity_filter(h, qx, qy, hc);
+        return face_of<false>(h, qx, qy, H, hc, ok);
+    }
+    bool in = true;
+    const Divisor<true> d(h + kEpsilon, in);
+    double c = d.of(hc, in);
+    const double u = d.of(qx), v = d.of(qy);
+    in &= wet_divisor(d.d) & calm(qx, u) & calm(qy, v);
+    const bool dry = (h == 0.0) & (hc == 0.0) & (fabs(qx) + fabs(qy) < 1e30);
+    ok &= in | dry;
+    c = (c > 0.0) ? c : 0.0;
+    qx = dry ? 0.0 : h * u;
+    qy = dry ? 0.0 : h * v;
+    hc = h * c;
+    Face5 f;
+    f.h = h;
+    f.H = H;
+    f.u = dry ? 0.0 : d.near(qx, u);
+    f.v = dry ? 0.0 : d.near(qy, v);
+    f.c = dry ? 0.0 : d.near(hc, c);
+    return f;
+}
+
+// avg, the van-Leer-type limiter (GPU/Reconstructor.cu:19-31): with a and b
+// of the same sign (a |b| + b |a|) / (|a| + |b|) is 2 a b / (a + b), every
+// operation rounding alike; of opposite sign its numerator is an exact zero.
+template <bool FAST>
+__device__ __forceinline__ double limit(double a, double b, bool &ok) {
+    if (!FAST) return limiter(a, b);
+    const double p = a * b, s = a + b;
+    const bool live = (p > 0.0) & (fabs(s) > kEpsilon);
+    const Divisor<true> d(live ? s : 1.0, ok);
+    ok &= mid(p) | !live;
+    return d.of(live ? p + p : 0.0);
+}
+
 // bedload (GPU/SedFlux.cuh:150-168), or the Grass law when selected; modu
 // is |u| as bedload() computes it.  The Ashida-Michiue product
 // K1*Q*max(O-OC,0)*max(sqrt(O)-sqrt(OC),0)*(h>HQB)*(h>5DS) has the sign of
@@ -142,75 +264,95 @@ __device__ __forceinline__ double bedload_flux(const Phys64 &P, double h, double
     return -qb;
 }
 
-// Cflux (GPU/SedFlux.cuh:171-179).  With the bedload switched off or a fixed
-// bed, F[3] = bedload * 0 is a zero with the sign of the bedload, i.e.
-// -copysign(0, u) (NaN when |u| is NaN); produced without evaluating it.
-__device__ __forceinline__ void phys_flux(const Phys64 &P, double h, double ux, double modu, double hc,
-                                          int fixed, double uy, double F[5]) {
-    F[0] = h * ux;
-    F[1] = F[0] * ux;
-    F[2] = F[0] * uy;
-    if (fixed != 0 && P.bedload != 0) F[3] = bedload_flux(P, h, ux, modu) * (double)fixed * (double)P.bedload;
-    else F[3] = isnan(modu) ? modu : -copysign(0.0, ux);
-    F[4] = hc * ux;
+// The bed component of Cflux (GPU/SedFlux.cuh:171-179) of a face with depth h
+// and velocity (u, v).  With the bedload switched off or a fixed bed it is
+// bedload * 0, a zero (NaN for a NaN velocity).
+__device__ __forceinline__ double bed_flux(const Phys64 &P, double h, double u, double v, bool moves) {
+    const double m2 = u * u + v * v;
+    if (isnan(m2)) return m2;
+    if (!moves) return 0.0;
+    return bedload_flux(P, h, u, dsqrt(m2)) * (double)P.bedload;
+}
+// bedload_flux without branches for the Ashida-Michiue law
+__device__ __forceinline__ double bed_flux_fast(const Phys64 &P, double h, double u, double v, bool &ok) {
+    const double m2 = u * u + v * v;
+    ok &= mid_or_zero(m2);
+    const double m = root(m2), O = P.Opar * m * m;
+    ok &= mid_or_zero(O);
+    const double K1 = Divisor<true>(m + kEpsilon, ok).of(17.0 * u, ok);
+    const double e = O - P.OC, f = root(O) - P.k.sqrt_OC;
+    const bool live = (e > 0.0) & (f > 0.0) & (h > P.HQB) & (h > P.k.DS5);
+    const double qb = K1 * P.Q * e * f;
+    return live ? -qb * (double)P.bedload : 0.0;
 }
 
-// One edge: RiemannSolver_Vols (GPU/VolumeSolver.cu:19-126) with the
-// rotation back of :129-152.  `a` is the state on the side the normal leaves
-// (index 0 in the reference), `b` the state it enters.  Dm is the
-// fluctuation into side a, Dp into side b, both in x/y components.
-__device__ __forceinline__ void edge_flux(const Phys64 &P, const State5 &a, const State5 &b, int nx, int ny,
-                                          int fixed, double Dm[5], double Dp[5]) {
-    // Both faces dry (h == 0 exactly, which also excludes NaN): every
-    // velocity, flux and depth below is a zero, the hydrostatic depths are
-    // max(-H + min(H_a, H_b), 0) = 0, both wave speeds are 0, so a0 = a1 = 0
-    // and all ten fluctuations evaluate to zeros.  They are returned as +0
-    // (the full evaluation can give -0 for some; a zero's sign does not
-    // reach any non-zero value of this scheme).  Dry land makes this the
-    // common edge of a coastal grid.
-    if (P.dry_skip && a.h == 0.0 && b.h == 0.0) {
-#pragma unroll
-        for (int i = 0; i < 5; i++) Dm[i] = Dp[i] = 0.0;
-        return;
-    }
-    const double dnx = (double)nx, dny = (double)ny;
-    double qlx = a.qx * dnx + a.qy * dny;
-    double qly = a.qy * dnx - a.qx * dny;
-    double qrx = b.qx * dnx + b.qy * dny;
-    double qry = b.qy * dnx - b.qx * dny;
-    double u0x, u0y, u1x, u1y, m0, m1;
-    velocity(a.h, qlx, qly, u0x, u0y, m0);
-    velocity(b.h, qrx, qry, u1x, u1y, m1);
-    double c0 = ddiv(a.hc, a.h + kEpsilon);
-    double c1 = ddiv(b.hc, b.h + kEpsilon);
-
+// One edge: RiemannSolver_Vols (GPU/VolumeSolver.cu:19-126) in the frame of
+// its normal: a is the face the normal leaves, b the one it enters, u / v
+// their velocities along n and along n turned left.  Dm is the fluctuation
+// into side a, Dp into side b, components (h, qn, qt, H, hc).
+template <bool FAST>
+__device__ __forceinline__ bool edge_flux(const Phys64 &P, const Face5 &a, const Face5 &b, int fixed, double Dm[5],
+                                          double Dp[5]) {
+    bool ok = true;
     // hydrostatic reconstruction (:37-40)
-    double zmH = fmin(a.H, b.H);
-    double h0 = fmax(a.h - a.H + zmH, 0.0);
-    double h1 = fmax(b.h - b.H + zmH, 0.0);
-    double q0x = u0x * h0, q0y = u0y * h0;
-    double q1x = u1x * h1, q1y = u1y * h1;
-    double hc0 = h0 * c0, hc1 = h1 * c1;
-    double deta = h1 - h0;
-
+    const double zmH = fmin(a.H, b.H);
+    double h0 = a.h - a.H + zmH, h1 = b.h - b.H + zmH;
+    h0 = (h0 > 0.0) ? h0 : 0.0;  // fmax(h0, 0)
+    h1 = (h1 > 0.0) ? h1 : 0.0;
+    const double deta = h1 - h0;
+    if (FAST && h0 == 0.0 && h1 == 0.0) {
+        // no water stands against either side (both faces dry, or water below
+        // the other side's bed): F and DU are zeros, and so is everything the
+        // finite wave speeds multiply.  Dry land makes this a common edge.
+        const double z = 0.0 * (a.u + a.v + a.c + b.u + b.v + b.c);
+#pragma unroll
+        for (int i = 0; i < 5; i++) Dm[i] = Dp[i] = z;
+        return true;
+    }
     double F0[5], F1[5];
-    phys_flux(P, h0, u0x, m0, hc0, fixed, u0y, F0);
-    phys_flux(P, h1, u1x, m1, hc1, fixed, u1y, F1);
+    // bed fluxes first: the only part with a branch
+    F0[3] = F1[3] = 0.0;
+    const bool moves = (fixed != 0) & (P.bedload != 0);
+    if (!FAST || (moves & (P.bedload_law != 0))) {
+        F0[3] = bed_flux(P, h0, a.u, a.v, moves);
+        F1[3] = bed_flux(P, h1, b.u, b.v, moves);
+    } else if (moves & !(P.still(a.u) & P.still(a.v) & P.still(b.u) & P.still(b.v))) {
+        F0[3] = bed_flux_fast(P, h0, a.u, a.v, ok);
+        F1[3] = bed_flux_fast(P, h1, b.u, b.v, ok);
+    }
+    const double hc0 = h0 * a.c, hc1 = h1 * b.c;
+    F0[0] = h0 * a.u;
+    F0[1] = F0[0] * a.u;
+    F0[2] = F0[0] * a.v;
+    F0[4] = hc0 * a.u;
+    F1[0] = h1 * b.u;
+    F1[1] = F1[0] * b.u;
+    F1[2] = F1[0] * b.v;
+    F1[4] = hc1 * b.u;
 
     // Roe average + wave-speed bounds (GPU/SedFlux.cuh:181-199)
-    double hm = 0.5 * (h0 + h1);
-    double s0q = dsqrt(h0), s1q = dsqrt(h1);
-    double umx = ddiv(s0q * u0x + s1q * u1x, s0q + s1q);
-    double SL = u0x - dsqrt(kG * h0);
-    double SR = u1x + dsqrt(kG * h1);
-    double cm = dsqrt(kG * hm);
-    SL = fmin(SL, umx - cm);
-    SR = fmax(SR, umx + cm);
+    const double hm = 0.5 * (h0 + h1);
+    if (FAST) ok &= mid_or_zero(h0) & mid_or_zero(h1);
+    const double s0q = root_of<FAST>(h0), s1q = root_of<FAST>(h1);
+    const double ghm = kG * hm;
+    double SL = a.u - root_of<FAST>(kG * h0), SR = b.u + root_of<FAST>(kG * h1);
+    const double cm = root_of<FAST>(ghm);
+    // two zero depths: 0/0, as in the reference, and the bounds below ignore it
+    const double umx = Divisor<FAST>(s0q + s1q, ok).of(s0q * a.u + s1q * b.u, ok);
+    const double sl = umx - cm, sr = umx + cm;
+    SL = (sl < SL) ? sl : SL;  // fmin / fmax of a possibly NaN second operand
+    SR = (sr > SR) ? sr : SR;
 
     double a0, a1;
-    if (SR - SL > kEpsilon) {
-        a0 = ddiv(SR * fabs(SL) - SL * fabs(SR), SR - SL);
-        a1 = ddiv(fabs(SR) - fabs(SL), SR - SL);
+    const double dS = SR - SL;
+    if (FAST) {
+        const Divisor<true> d(dS, ok);
+        ok &= dS > kEpsilon;
+        a0 = d.of(SR * fabs(SL) - SL * fabs(SR), ok);
+        a1 = d.of(fabs(SR) - fabs(SL), ok);
+    } else if (dS > kEpsilon) {
+        a0 = ddiv(SR * fabs(SL) - SL * fabs(SR), dS);
+        a1 = ddiv(fabs(SR) - fabs(SL), dS);
     } else {
         a0 = fmax(fabs(SL), fabs(SR));
         a1 = 0.0;
@@ -219,38 +361,24 @@ __device__ __forceinline__ void edge_flux(const Phys64 &P, const State5 &a, cons
     double df[5], DU[5];
 #pragma unroll
     for (int i = 0; i < 5; i++) df[i] = F1[i] - F0[i];
-    df[1] += kG * hm * deta;
-    DU[0] = h1 - h0;
-    DU[1] = q1x - q0x;
-    DU[2] = q1y - q0y;
-    DU[3] = b.H - a.H;
+    df[1] += ghm * deta;
+    DU[0] = deta;
+    DU[1] = F1[0] - F0[0];  // q = u h, the mass flux
+    DU[2] = b.v * h1 - a.v * h0;
+    DU[3] = 0.0;  // replaced by the upwinded bed component below
     DU[4] = hc1 - hc0;
-    double s0 = sgn(b.H - a.H);
-    double s1 = sgn(df[3]);
-    double s2 = sgn(a1);
-    if (fabs(s0) > kEpsilon) s1 = s1 * s0;  // s0 is +-1: s1/s0 == s1*s0 exactly
-    else s1 = 0.0;
+    const int s0 = sgn(b.H - a.H), s2 = sgn(a1);
+    const int s1 = sgn(df[3]) * s0;  // s1 / s0 for s0 = +-1, 0 for s0 = 0
     double vis[5];
 #pragma unroll
     for (int i = 0; i < 5; i++) vis[i] = a0 * DU[i] + a1 * df[i];
-    if (s2 == s1) vis[3] = a1 * df[3];
-    else vis[3] = -a1 * df[3];
-    double m[5], p[5];
+    vis[3] = (s2 == s1) ? a1 * df[3] : -a1 * df[3];
 #pragma unroll
     for (int i = 0; i < 5; i++) {
-        m[i] = 0.5 * (df[i] - vis[i]) + F0[i];
-        p[i] = 0.5 * (df[i] + vis[i]) - F1[i];
+        Dm[i] = 0.5 * (df[i] - vis[i]) + F0[i];
+        Dp[i] = 0.5 * (df[i] + vis[i]) - F1[i];
     }
-    Dm[0] = m[0];
-    Dm[1] = (dnx * m[1] - dny * m[2]);
-    Dm[2] = (dny * m[1] + dnx * m[2]);
-    Dm[3] = m[3];
-    Dm[4] = m[4];
-    Dp[0] = p[0];
-    Dp[1] = (dnx * p[1] - dny * p[2]);
-    Dp[2] = (dny * p[1] + dnx * p[2]);
-    Dp[3] = p[3];
-    Dp[4] = p[4];
+    return ok;
 }
 
 // MUSCL-Hancock half-step predictor (RK == 0, GPU/Reconstructor.cu:280-342)
@@ -358,6 +486,24 @@ __device__ __forceinline__ double cfl_dt(const Phys64 &P, double h, double qx, d
     double lx = fabs(ux) + cg;
     double ly = fabs(uy) + cg;
     return P.CFL * 0.5 * fmin(ddiv_inf(P.dx, lx), ddiv_inf(P.dy, ly));
+}
+
+// The same of a wet cell from the velocity of its filtered state.  On square
+// cells the smaller of dx / lx and dy / ly is dx over the larger speed (the
+// rounded quotient does not increase with the divisor).
+__device__ __forceinline__ bool cfl_dt_fast(const Phys64 &P, const Face5 &f, double &dt) {
+    bool ok = mid(f.h);
+    const double cg = root(kG * f.h);
+    const double lx = fabs(f.u) + cg, ly = fabs(f.v) + cg;
+    double q;
+    if (P.dx == P.dy) {
+        q = Divisor<true>((lx > ly) ? lx : ly, ok).of(P.dx, ok);
+    } else {
+        const double qx = Divisor<true>(lx, ok).of(P.dx, ok), qy = Divisor<true>(ly, ok).of(P.dy, ok);
+        q = (qx < qy) ? qx : qy;
+    }
+    dt = P.CFL * 0.5 * q;
+    return ok;
 }
 
 }  // namespace tsu

@@ -176,6 +176,9 @@ static void fill_phys(TsuSolver *s) {
     P.inv_dx = 1.0 / p->dx;  // GPU/main_TSUNER.cu:43-44
     P.inv_dy = 1.0 / p->dy;
     P.k = s->hconsts;
+    P.inv_vs = 1.0 / s->hconsts.vs;
+    const double rest = std::sqrt(0.495 * p->OC / p->Opar);
+    P.still_hi = (rest > 0.0 && rest < 1e30) ? hi32(rest) : 0u;
     P.npx = p->npx;
     P.npy = p->npy;
     P.order = sw->order;
@@ -284,7 +287,7 @@ static int create_solver(TsuSolver **out, const SimParams *pg, const TsuSwitches
     s->st = s->own_st;
     if (e == cudaSuccess) e = cudaEventCreate(&s->e0);
     if (e == cudaSuccess) e = cudaEventCreate(&s->e1);
-    if (e == cudaSuccess) e = s->fp32 ? stage32_prepare() : stage64_prepare();
+    if (e == cudaSuccess) e = s->fp32 ? stage32_prepare() : stage64_prepare(p->npx, p->npy);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->A, 0, 5 * pl, s->st);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->B, 0, 5 * pl, s->st);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->mask, 1, (size_t)s->plane, s->st);
@@ -308,7 +311,7 @@ static int create_solver(TsuSolver **out, const SimParams *pg, const TsuSwitches
             // the maps cover every stored row (ghost rows included)
             const double *ext[3] = {(const double *)s->hmax, (const double *)s->bmin, (const double *)s->eta};
             s->tma = stage64_tma_maps((const double *)s->A, (const double *)s->B, s->mask, ext, s->pitch, s->plane,
-                                      p->npx, nstore, &s->tmA, &s->tmB, &s->tmM, &s->tmO, s->tmE);
+                                      p->npx, nstore, &s->tmA, &s->tmB, &s->tmM, &s->tmO, s->tmE, p->npy);
         }
     }
     if (e != cudaSuccess) {

@@ -24,6 +24,13 @@
 // Phases 3 and 4 each have a single call site of the reconstruction and of
 // the Riemann solver (boundary cases only select operands), which keeps the
 // kernel body small enough for the instruction cache.
+// What bounds it: the dependent FP64 instructions of ~50 divisions and ~20
+// roots per cell and stage.  They are evaluated without branches and with
+// shared reciprocals (ieee64.h), each phase with one test that sends the
+// operands it cannot take to a general form of the same formulas.  4096^2,
+// the N-wave entering still water, 2 steps: 12.1 -> 9.6 ms; 1021 x 773 with
+// currents everywhere, 4 steps: 1350 -> 943 us (FP64 pipe 34 -> 46 % busy, 117
+// -> 87 warp instructions per cell in the first stage).
 #include <cuda_runtime.h>
 
 #include <cstdlib>
@@ -47,7 +54,8 @@ struct Tile {
     static constexpr int kSV = 5 * PS, kSUC = 3 * PS, kFlux = 20 * TY * TX;
     static constexpr int kRegA = (kSV + kSUC) > kFlux ? (kSV + kSUC) : kFlux;
     static constexpr int kFx = 10 * TY * FXW, kFy = 10 * FYH * TX, kDeta = 2 * TY * TX, kRed = NT / 32;
-    static constexpr int kDoubles = kRegA + kFx + kFy + kDeta + kRed;
+    static constexpr int kSeam = 4 * (TX + TY);  // seam discharges (periodic grids with a boundary series)
+    static constexpr int kDoubles = kRegA + kFx + kFy + kDeta + kRed + kSeam;
     // the 1-byte mask: rows of MLX = TX + 32 cells starting 16 left of the
     // tile (a 16-byte aligned TMA origin for bytes), 128-byte aligned
     static constexpr int MHX = 16, MLX = TX + 2 * MHX, MPS = MLX * LY;
@@ -74,10 +82,10 @@ __device__ __forceinline__ int wrap_clamp(int g, int n, bool periodic) {
 // :124-194 (x) / :207-271 (y).  c/l/r index the centre and its two
 // neighbours in the smem tile (plane stride PS).  Returns the two faces
 // (minus side, plus side) before the state filter and the hydrostatic slope
-// deta.
-template <int PS>
+// deta; `ok` as in physics64.cuh.
+template <int PS, bool FAST>
 __device__ __forceinline__ void reconstruct_dir(const double *sV, const double *sUC, int c, int l, int r,
-                                                State5 &fm, State5 &fp, double &deta) {
+                                                State5 &fm, State5 &fp, double &deta, bool &ok) {
     const double hi = sV[c], Hi = sV[3 * PS + c];
     const double hl = sV[l], Hl = sV[3 * PS + l];
     const double hr = sV[r], Hr = sV[3 * PS + r];
@@ -87,16 +95,18 @@ __device__ __forceinline__ void reconstruct_dir(const double *sV, const double *
     const double urx = sUC[r], ury = sUC[PS + r];
 
     double dl = hi - hl, dr = hr - hi;
-    double dh = limiter(dl, dr);
+    double dh = limit<FAST>(dl, dr, ok);
     if (0.5 * fabs(dh) > hi) dh = 2.0 * hi * sgn(dh);
     fm.h = hi - 0.5 * dh;
     fp.h = hi + 0.5 * dh;
 
+    // pos(x) = fmax(x, 0)
+    auto pos = [](double x) { return (x > 0.0) ? x : 0.0; };
     double zm = fmin(Hl, Hi);
-    dl = fmax(hi - Hi + zm, 0.0) - fmax(hl - Hl + zm, 0.0);
+    dl = pos(hi - Hi + zm) - pos(hl - Hl + zm);
     zm = fmin(Hr, Hi);
-    dr = fmax(hr - Hr + zm, 0.0) - fmax(hi - Hi + zm, 0.0);
-    deta = limiter(dl, dr);
+    dr = pos(hr - Hr + zm) - pos(hi - Hi + zm);
+    deta = limit<FAST>(dl, dr, ok);
     double dz = dh - deta;
     fm.H = Hi - 0.5 * dz;
     fp.H = Hi + 0.5 * dz;
@@ -104,45 +114,163 @@ __device__ __forceinline__ void reconstruct_dir(const double *sV, const double *
     const double qxi = sV[PS + c], qyi = sV[2 * PS + c];
     dl = uix - ulx;
     dr = urx - uix;
-    double du = limiter(dl, dr);
+    double du = limit<FAST>(dl, dr, ok);
     double dq = hi * du + uix * dh;
     fm.qx = qxi - 0.5 * dq;
     fp.qx = qxi + 0.5 * dq;
     dl = uiy - uly;
     dr = ury - uiy;
-    du = limiter(dl, dr);
+    du = limit<FAST>(dl, dr, ok);
     dq = hi * du + uiy * dh;
     fm.qy = qyi - 0.5 * dq;
     fp.qy = qyi + 0.5 * dq;
 
     dl = ci - cl;
     dr = cr - ci;
-    du = limiter(dl, dr);
+    du = limit<FAST>(dl, dr, ok);
     fm.hc = (ci - 0.5 * du) * fm.h;
     fp.hc = (ci + 0.5 * du) * fp.h;
 }
 
-__device__ __forceinline__ void filter5(State5 &s) { positivity_filter(s.h, s.qx, s.qy, s.hc); }
-
-__device__ __forceinline__ void put5(double *base, int stride, const State5 &s) {
+__device__ __forceinline__ void put5(double *base, int stride, const Face5 &s) {
     base[0] = s.h;
-    base[stride] = s.qx;
-    base[2 * stride] = s.qy;
+    base[stride] = s.u;
+    base[2 * stride] = s.v;
     base[3 * stride] = s.H;
-    base[4 * stride] = s.hc;
+    base[4 * stride] = s.c;
 }
-__device__ __forceinline__ State5 get5(const double *base, int stride) {
-    State5 s;
+__device__ __forceinline__ Face5 get5(const double *base, int stride) {
+    Face5 s;
     s.h = base[0];
-    s.qx = base[stride];
-    s.qy = base[2 * stride];
+    s.u = base[stride];
+    s.v = base[2 * stride];
     s.H = base[3 * stride];
-    s.hc = base[4 * stride];
+    s.c = base[4 * stride];
     return s;
 }
-__device__ __forceinline__ void put5a(double *base, int stride, const double D[5]) {
+// A face in the frame of the normal (0, 1): velocity along it and along it
+// turned left (GPU/VolumeSolver.cu:24-27).  Faces along y are kept this way.
+__device__ __forceinline__ Face5 to_y(const Face5 &f) {
+    Face5 r = f;
+    r.u = f.v;
+    r.v = -f.u;
+    return r;
+}
+template <bool FAST>
+__device__ __forceinline__ Face5 filtered(State5 &s, bool &ok) {
+    return filter_face<FAST>(s.h, s.qx, s.qy, s.H, s.hc, ok);
+}
+
+// Both faces of a cell along one direction, filtered, to shared memory.
+// False (FAST only): an operand was out of range and what was stored is not
+// valid.  qplus / qminus (may be null): the discharges of the plus-side face
+// normal to its edge and of the minus-side face along it, for the periodic
+// seam (ydir: the direction is y).
+template <int PS, bool FAST>
+__device__ __forceinline__ bool make_faces(const double *sV, const double *sUC, int c, int step, double *dst,
+                                           int fstride, int side, double *deta_out, double *qplus = nullptr,
+                                           double *qminus = nullptr) {
+    bool ok = true;
+    State5 m, p;
+    double deta;
+    reconstruct_dir<PS, FAST>(sV, sUC, c, c - step, c + step, m, p, deta, ok);
+    Face5 fm = filtered<FAST>(m, ok), fp = filtered<FAST>(p, ok);  // GPU/Reconstructor.cu:344-348
+    if (step != 1) {
+        fm = to_y(fm);
+        fp = to_y(fp);
+    }
+    put5(dst, fstride, fm);
+    put5(dst + side, fstride, fp);
+    if (deta_out) *deta_out = deta;
+    if (qplus) *qplus = (step != 1) ? p.qy : p.qx;
+    if (qminus) *qminus = (step != 1) ? m.qx : m.qy;
+    return ok;
+}
+template <int PS>
+__device__ __noinline__ void make_faces_any(const double *sV, const double *sUC, int c, int step, double *dst,
+                                            int fstride, int side, double *deta_out, double *qplus, double *qminus) {
+    make_faces<PS, false>(sV, sUC, c, step, dst, fstride, side, deta_out, qplus, qminus);
+}
+
+// The fluctuations of one edge, in its frame, to the cells on its two sides
+// (null: the side is not in the tile).
+template <bool FAST>
+__device__ __forceinline__ bool put_edge(const Phys64 &P, const Face5 &a, const Face5 &b, int fixed, double *outM,
+                                         double *outP, int FS) {
+    double Dm[5], Dp[5];
+    const bool ok = edge_flux<FAST>(P, a, b, fixed, Dm, Dp);
 #pragma unroll
-    for (int f = 0; f < 5; f++) base[f * stride] = D[f];
+    for (int f = 0; f < 5; f++) {
+        if (outM) outM[f * FS] = Dm[f];
+        if (outP) outP[f * FS] = Dp[f];
+    }
+    return ok;
+}
+__device__ __noinline__ void put_edge_any(const Phys64 &P, Face5 a, Face5 b, int fixed, double *outM, double *outP,
+                                          int FS) {
+    put_edge<false>(P, a, b, fixed, outM, outP, FS);
+}
+
+// Friction (GPU/Reconstructor.cu:33-55) on the momentum (k1, k2) and the
+// erosion/deposition rate phi (:57-88), from U^n = v0; one velocity
+// evaluation serves both.
+template <bool FAST>
+__device__ __forceinline__ bool sources(const Phys64 &P, double dt, const double v0[5], double &k1, double &k2,
+                                        double &phi) {
+    bool ok = true;
+    double ux, uy, modu;
+    const Divisor<FAST> d0(v0[0] + kEpsilon, ok);
+    if (FAST) {
+        ux = d0.of(v0[1]);
+        uy = d0.of(v0[2]);
+        const double m2 = ux * ux + uy * uy;
+        ok &= wet_divisor(d0.d) & calm(v0[1], ux) & calm(v0[2], uy) & mid_or_zero(m2);
+        modu = root(m2);
+    } else {
+        velocity(v0[0], v0[1], v0[2], ux, uy);
+        modu = dsqrt(ux * ux + uy * uy);
+    }
+    if (!FAST && P.manning) {  // GPU/Reconstructor.cu:47-50 as written (multiplies)
+        const double cm = dt * P.FR * P.FR * modu / pow(v0[0], 4.0 / 3.0);
+        k1 *= cm;
+        k2 *= cm;
+    } else {
+        const double cf = d0.of(dt * P.FR * modu, ok);
+        const Divisor<FAST> d1(1.0 + cf, ok);
+        k1 = d1.of(k1, ok);
+        k2 = d1.of(k2, ok);
+    }
+    const double c = Divisor<FAST>(v0[0] + P.eps_h, ok).of(v0[4], ok);
+    const double A = P.k.A_er * (modu * P.k.sqrt_FR);
+    double Z;
+    if (FAST) {
+        ok &= mid_or_zero(A);
+        Z = quot(A, P.k.vs, P.inv_vs);
+    } else {
+        Z = ddiv(A, P.k.vs);
+    }
+    const double Z5 = Z * Z * Z * Z * Z;
+    const double Es = Divisor<FAST>(1 + 4.3e-7 * Z5, ok).of(1.3e-7 * Z5, ok);
+    double Fe = P.k.VP * Es;
+    if (Fe > 0.1) Fe = 0.1;
+    Fe = Fe * (double)(Fe > 0.0);
+    double Cb = P.k.K_dep * c;
+    double Fd = P.k.vs * Cb;
+    if (Fd > 0.1) Fd = 0.1;
+    Fd = Fd * (double)(Fd > 0.0);
+    phi = (Fe - Fd) * (double)P.suspension;
+    return ok;
+}
+struct Sources {
+    double k1, k2, phi;
+};
+__device__ __noinline__ Sources sources_any(const Phys64 &P, double dt, State5 v, double k1, double k2) {
+    const double v0[5] = {v.h, v.qx, v.qy, v.H, v.hc};
+    Sources r;
+    r.k1 = k1;
+    r.k2 = k2;
+    sources<false>(P, dt, v0, r.k1, r.k2, r.phi);
+    return r;
 }
 
 // RK0: MUSCL-Hancock (RK == 0 of the reference): one stage per step
@@ -162,7 +290,7 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
     constexpr bool PINGPONG = (ORDER == 1) || RK0;
     constexpr bool LATE = (OWN >= 1);
     using T = Tile<TX, TY, NTHR>;
-    constexpr int NT = T::NT, LX = T::LX, LY = T::LY, PS = T::PS, FXW = T::FXW, FYH = T::FYH;
+    constexpr int NT = T::NT, LX = T::LX, PS = T::PS, FXW = T::FXW, FYH = T::FYH;
     constexpr int MHX = T::MHX, MLX = T::MLX;
     extern __shared__ __align__(16) double smem_raw[];
     double *smem = smem_align<128>(smem_raw);
@@ -176,6 +304,7 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
     double *sFy = sFx + T::kFx;         // [2][5][FYH][TX]
     double *sDeta = sFy + T::kFy;       // [2][TY][TX]
     double *sRed = sDeta + T::kDeta;    // [NT/32]
+    double *sSeam = sRed + T::kRed;     // [2][2 TY + 2 TX]
     unsigned char *sM = reinterpret_cast<unsigned char *>(smem) + T::kMaskOff;  // [LY][MLX], tile at column MHX
     __shared__ int sLast;
 
@@ -295,20 +424,31 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
     }
 
     // ---- phase 2: per-cell velocity and concentration
-    if (ORDER == 2) {
-        for (int idx = tid; idx < PS; idx += NT) {
-            double h = sV[idx];
-            double ux, uy;
-            velocity(h, sV[PS + idx], sV[2 * PS + idx], ux, uy);
-            sUC[idx] = ux;
-            sUC[PS + idx] = uy;
-            sUC[2 * PS + idx] = ddiv(sV[4 * PS + idx], h + kEpsilon);
-        }
-        __syncthreads();
+    for (int idx = tid; idx < PS; idx += NT) {
+        const double h = sV[idx], qx = sV[PS + idx], qy = sV[2 * PS + idx], hc = sV[4 * PS + idx];
+        bool ok = wet_divisor(h);
+        Face5 f;
+        if (ok) f = face_of<true>(h, qx, qy, 0.0, hc, ok);
+        if (!ok) f = face_of<false>(h, qx, qy, 0.0, hc, ok);
+        sUC[idx] = f.u;
+        sUC[PS + idx] = f.v;
+        sUC[2 * PS + idx] = f.c;
     }
+    __syncthreads();
+
+    // Periodic grids with an expired boundary series mirror the discharge of the
+    // seam's low-side face into its high-side face (phase 4).  The faces do not
+    // hold discharges, so those of the edges at the grid's two ends are kept
+    // aside: which = 0 the low-side face's normal discharge, 1 the high-side
+    // face's transverse one; k: row or column of the tile; e: global edge index.
+    const bool seam_q = periodic && P.read_files;
+    auto seam_slot = [&](bool vert, int which, int k, int e) -> double * {
+        const int end = vert ? npx : P.ny_glob;
+        if (e != 0 && e != end) return nullptr;
+        return sSeam + which * T::kSeam / 2 + (vert ? 0 : 2 * TY) + (e == 0 ? 0 : (vert ? TY : TX)) + k;
+    };
 
     // ---- phase 3: faces (one reconstruction call site)
-    constexpr int NXI = FXW * TY, NYI = TX * FYH;
     if (RK0 && ORDER == 2) {
         // MUSCL-Hancock: the predictor needs all four faces of a cell, so an
         // item is a cell -- the tile, then its halo columns -1 / TX (x faces
@@ -331,22 +471,27 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
             const int c = (ly + 2) * LX + (lx + 2);
             State5 L, R, D, U;
             double detx, dety;
-            reconstruct_dir<PS>(sV, sUC, c, c - 1, c + 1, L, R, detx);
-            reconstruct_dir<PS>(sV, sUC, c, c - LX, c + LX, D, U, dety);
+            bool ok = true;
+            reconstruct_dir<PS, false>(sV, sUC, c, c - 1, c + 1, L, R, detx, ok);
+            reconstruct_dir<PS, false>(sV, sUC, c, c - LX, c + LX, D, U, dety, ok);
             hancock_predictor(P, dt, sV[c], detx, dety, L, R, D, U);
-            filter5(L);
-            filter5(R);
-            filter5(U);
-            filter5(D);
             if (ly >= 0 && ly < TY) {
                 double *dst = sFx + ly * FXW + (lx + 1);
-                put5(dst, TY * FXW, L);
-                put5(dst + 5 * TY * FXW, TY * FXW, R);
+                put5(dst, TY * FXW, filtered<false>(L, ok));
+                put5(dst + 5 * TY * FXW, TY * FXW, filtered<false>(R, ok));
+                if (seam_q) {
+                    if (double *q = seam_slot(true, 0, ly, x0 + lx + 1)) *q = R.qx;
+                    if (double *q = seam_slot(true, 1, ly, x0 + lx)) *q = L.qy;
+                }
             }
             if (lx >= 0 && lx < TX) {
                 double *dst = sFy + (ly + 1) * TX + lx;
-                put5(dst, FYH * TX, D);
-                put5(dst + 5 * FYH * TX, FYH * TX, U);
+                put5(dst, FYH * TX, to_y(filtered<false>(D, ok)));
+                put5(dst + 5 * FYH * TX, FYH * TX, to_y(filtered<false>(U, ok)));
+                if (seam_q) {
+                    if (double *q = seam_slot(false, 0, lx, P.j0 + y0 + ly + 1)) *q = U.qy;
+                    if (double *q = seam_slot(false, 1, lx, P.j0 + y0 + ly)) *q = D.qx;
+                }
             }
             if (lx >= 0 && lx < TX && ly >= 0 && ly < TY) {
                 sDeta[ly * TX + lx] = detx;
@@ -354,98 +499,123 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
             }
         }
     }
-    for (int item = tid; item < ((RK0 && ORDER == 2) ? 0 : NXI + NYI); item += NT) {
-        int c, step, fstride, side, didx = -1;
-        double *dst;
-        if (item < NXI) {
-            int r = item / FXW, cx = item - r * FXW;  // tile col cx-1
-            c = (r + 2) * LX + (cx + 1);
-            step = 1;
-            dst = sFx + r * FXW + cx;
-            fstride = TY * FXW;
-            side = 5 * TY * FXW;
-            int tc = cx - 1;
-            if (tc >= 0 && tc < TX) didx = r * TX + tc;
+    // Otherwise a warp's item is 32 faces: the x faces of RPW tile rows, the y
+    // faces of RPW rows (one halo row on each side included), or part of the x
+    // faces of the halo columns (two per row), last because it is not full.
+    // 19 items for 10 warps: two rounds.
+    constexpr int RPW = 32 / TX, WX = TY / RPW, WY = (FYH + RPW - 1) / RPW, WF = (2 * TY + 31) / 32;
+    static_assert(32 % TX == 0 && TY % RPW == 0, "tile rows per warp");
+    const int warp = tid >> 5, lr = (tid & 31) / TX, lc = (tid & 31) % TX;
+    for (int item = warp; item < ((RK0 && ORDER == 2) ? 0 : WX + WY + WF); item += NT / 32) {
+        const bool xi = item < WX || item >= WX + WY;
+        int lx, ly;  // the cell, in tile coordinates
+        if (item < WX) {
+            lx = lc;
+            ly = item * RPW + lr;
+        } else if (xi) {
+            const int k = (item - WX - WY) * 32 + (tid & 31);
+            lx = (k & 1) ? TX : -1;
+            ly = k >> 1;
+            if (ly >= TY) continue;
         } else {
-            int it = item - NXI;
-            int ry = it / TX, cc = it - ry * TX;  // tile row ry-1
-            c = (ry + 1) * LX + (cc + 2);
-            step = LX;
-            dst = sFy + ry * TX + cc;
-            fstride = FYH * TX;
-            side = 5 * FYH * TX;
-            int tr = ry - 1;
-            if (tr >= 0 && tr < TY) didx = TY * TX + tr * TX + cc;
+            lx = lc;
+            ly = (item - WX) * RPW + lr - 1;
+            if (ly > TY) continue;
         }
-        State5 fm, fp;
+        const int c = (ly + 2) * LX + (lx + 2), step = xi ? 1 : LX;
+        double *dst = xi ? sFx + ly * FXW + (lx + 1) : sFy + (ly + 1) * TX + lx;
+        const int fstride = xi ? TY * FXW : FYH * TX, side = 5 * fstride;
+        int didx = -1;  // the cell is in the tile
+        if (item < WX) didx = ly * TX + lx;
+        else if (!xi && ly >= 0 && ly < TY) didx = TY * TX + ly * TX + lx;
+        double *qplus = nullptr, *qminus = nullptr;
+        if (seam_q) {  // the cell's plus face is at the edge after it, its minus face at the edge before
+            const int k = xi ? ly : lx, e = xi ? x0 + lx : P.j0 + y0 + ly;
+            qplus = seam_slot(xi, 0, k, e + 1);
+            qminus = seam_slot(xi, 1, k, e);
+        }
         if (ORDER == 2) {
-            double deta;
             if (P.dry_skip && sV[c] == 0.0 && sV[c - step] == 0.0 && sV[c + step] == 0.0) {
                 // a dry stencil: every slope is avg(0, 0) = 0, so both faces
                 // are (0, q_i, 0, H_i, 0 * c) before the filter and (0, 0, 0,
                 // H_i, 0) after it (zeros up to their sign), and deta = 0
-                fm.h = fm.qx = fm.qy = fm.hc = 0.0;
-                fm.H = sV[3 * PS + c];
-                fp = fm;
-                deta = 0.0;
+                Face5 f;
+                f.h = f.u = f.v = f.c = 0.0;
+                f.H = sV[3 * PS + c];
+                put5(dst, fstride, f);
+                put5(dst + side, fstride, f);
+                if (didx >= 0) sDeta[didx] = 0.0;
+                if (qplus) *qplus = 0.0;
+                if (qminus) *qminus = 0.0;
             } else {
-                reconstruct_dir<PS>(sV, sUC, c, c - step, c + step, fm, fp, deta);
-                filter5(fm);  // GPU/Reconstructor.cu:344-348
-                filter5(fp);
+                double *deta = (didx >= 0) ? sDeta + didx : nullptr;
+                if (seam_q || !make_faces<PS, true>(sV, sUC, c, step, dst, fstride, side, deta))
+                    make_faces_any<PS>(sV, sUC, c, step, dst, fstride, side, deta, qplus, qminus);
             }
-            if (didx >= 0) sDeta[didx] = deta;
         } else {  // first order: faces are the cell values (GPU/Reconstructor.cu:99-107)
-            fm = get5(sV + c, PS);
-            fp = fm;
+            Face5 f;
+            f.h = sV[c];
+            f.u = sUC[c];
+            f.v = sUC[PS + c];
+            f.H = sV[3 * PS + c];
+            f.c = sUC[2 * PS + c];
+            if (!xi) f = to_y(f);
+            put5(dst, fstride, f);
+            put5(dst + side, fstride, f);
+            if (qplus) *qplus = sV[(step == 1 ? 1 : 2) * PS + c];
+            if (qminus) *qminus = sV[(step == 1 ? 2 : 1) * PS + c];
         }
-        put5(dst, fstride, fm);
-        put5(dst + side, fstride, fp);
     }
     __syncthreads();
 
     // ---- phase 4: edges (each once per tile, one Riemann call site)
     const bool series_on = !inner && P.read_files && (t < A.tCC[A.timeCC - 2]);
-    constexpr int NV = (TX + 1) * TY, NH = TX * (TY + 1);
-    constexpr int FS = TY * TX;  // flux plane stride; planes FL, FR, FD, FU
-    for (int item = tid; item < NV + NH; item += NT) {
-        State5 a, b;
-        int nx, ny, fixed, seg = 0;
-        bool bnd = false, seam = false, vert;
+    constexpr int FS = TY * TX;  // flux plane stride; planes FL, FR, FD, FU, each in its edge's frame
+    // A warp's item is 32 edges: the east edges of RPW tile rows, the RPW rows
+    // of horizontal edges, or west edges of the tile (TY in all), last.
+    constexpr int WH = (TY + 1 + RPW - 1) / RPW, WW = (TY + 31) / 32;
+    for (int item = warp; item < WX + WH + WW; item += NT / 32) {
+        const bool vert = item < WX || item >= WX + WH;
+        int r, e, c;  // vertical edge e (0..TX) of row r, or horizontal edge e (0..TY) of column c
+        if (item < WX) {
+            r = item * RPW + lr;
+            e = lc + 1;
+            c = 0;
+        } else if (vert) {
+            r = (item - WX - WH) * 32 + (tid & 31);
+            e = c = 0;
+            if (r >= TY) continue;
+        } else {
+            r = 0;
+            e = (item - WX) * RPW + lr;
+            c = lc;
+            if (e > TY) continue;
+        }
+        Face5 a, b;
+        int n = 1, fixed, seg = 0;
+        bool bnd = false, seam = false;
         double *outM = nullptr, *outP = nullptr;
         if (inner) {  // interior edges only (uniform per tile): no bounds or boundary cases
-            if (item < NV) {
-                vert = true;
-                nx = 1;
-                ny = 0;
-                const int r = item / (TX + 1), e = item - r * (TX + 1);
+            if (vert) {
                 a = get5(sFx + (5 * TY + r) * FXW + e, TY * FXW);
                 b = get5(sFx + r * FXW + (e + 1), TY * FXW);
                 fixed = (int)sM[(r + 2) * MLX + e + 1 + (MHX - 2)] * (int)sM[(r + 2) * MLX + e + 2 + (MHX - 2)];
                 if (e >= 1) outM = sFlux + 1 * 5 * FS + r * TX + (e - 1);
                 if (e < TX) outP = sFlux + 0 * 5 * FS + r * TX + e;
             } else {
-                vert = false;
-                nx = 0;
-                ny = 1;
-                const int it = item - NV;
-                const int e = it / TX, c = it - e * TX;
                 a = get5(sFy + (5 * FYH + e) * TX + c, FYH * TX);
                 b = get5(sFy + (e + 1) * TX + c, FYH * TX);
                 fixed = (int)sM[(e + 1) * MLX + c + 2 + (MHX - 2)] * (int)sM[(e + 2) * MLX + c + 2 + (MHX - 2)];
                 if (e >= 1) outM = sFlux + 3 * 5 * FS + (e - 1) * TX + c;
                 if (e < TY) outP = sFlux + 2 * 5 * FS + e * TX + c;
             }
-        } else if (item < NV) {
-            vert = true;
-            const int r = item / (TX + 1), e = item - r * (TX + 1);
+        } else if (vert) {
             const int ex = x0 + e, ey = y0 + r;
             if (ey >= npy || ex > npx) continue;
             const int ly = r + 2;
             // R face of tile col e-1 is sFx col e; L face of tile col e is col e+1
             const double *Rf = sFx + (5 * TY + r) * FXW + e;
             const double *Lf = sFx + r * FXW + (e + 1);
-            nx = 1;
-            ny = 0;
             const int J = P.j0 + ey;  // the global row (boundary-series segments)
             if (periodic && (ex == 0 || ex == npx)) {  // seam: GPU/VolumeSolver.cu:262-275,289-298
                 a = get5(Rf, TY * FXW);
@@ -457,7 +627,7 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
                 if (e < TX) outP = sFlux + 0 * 5 * FS + r * TX + e;
             } else if (ex == 0) {  // west: GPU/VolumeSolver.cu:233-258
                 a = get5(Lf, TY * FXW);
-                nx = -1;
+                n = -1;
                 fixed = sM[ly * MLX + e + 2 + (MHX - 2)];
                 bnd = true;
                 seg = 2 * npx + P.ny_glob + J;
@@ -476,16 +646,11 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
                 if (e < TX) outP = sFlux + 0 * 5 * FS + r * TX + e;
             }
         } else {
-            vert = false;
-            const int it = item - NV;
-            const int e = it / TX, c = it - e * TX;
             const int ex = x0 + c, ey = y0 + e;
             if (ex >= npx || ey > npy) continue;
             // U face of tile row e-1 is sFy row e; D face of tile row e is row e+1
             const double *Uf = sFy + (5 * FYH + e) * TX + c;
             const double *Df = sFy + (e + 1) * TX + c;
-            nx = 0;
-            ny = 1;
             // the grid's own south / north boundary (a slab's other edges are
             // interior edges, their far side in the ghost rows)
             const int J = P.j0 + ey;
@@ -500,7 +665,7 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
                 if (e < TY) outP = sFlux + 2 * 5 * FS + e * TX + c;
             } else if (south) {  // south: GPU/VolumeSolver.cu:324-349
                 a = get5(Df, FYH * TX);
-                ny = -1;
+                n = -1;
                 fixed = sM[(e + 2) * MLX + c + 2 + (MHX - 2)];
                 bnd = true;
                 seg = ex;
@@ -521,32 +686,60 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
         }
         if (bnd) {  // ghost = copy, wall mirror of the normal momentum
             b = a;
-            if (P.wbc == 1) {
-                if (vert) b.qx = -a.qx;
-                else b.qy = -a.qy;
-            }
+            if (P.wbc == 1) b.u = -a.u;
         }
         if ((bnd || seam) && P.read_files) {  // CC series while active, then wall
-            if (series_on) series_state(A.CC, A.tCC, t, npx, P.ny_glob, seg, b);
-            else if (vert) b.qx = -a.qx;
-            else b.qy = -a.qy;
-        }
-        double Dm[5], Dp[5];
-        edge_flux(P, a, b, nx, ny, fixed, Dm, Dp);
-        if (outM) put5a(outM, FS, Dm);
-        if (outP) put5a(outP, FS, Dp);
-    }
-    __syncthreads();
-
-    if (own_tma) {  // the owned cells' U^n and extrema have landed (bounded wait)
-        const bool ok = mbar_wait_first(&sBarOwn, 0);
-        if (__syncthreads_or(!ok)) {
-            if (tid == 0) {
-                A.scal[SC_ERR] = 1.0;
-                mbar_wait(&sBarOwn, 0);
+            if (series_on) {
+                State5 g;
+                series_state(A.CC, A.tCC, t, npx, P.ny_glob, seg, g);
+                bool ok = true;
+                b = face_of<false>(g.h, g.qx, g.qy, g.H, g.hc, ok);
+                if (!vert) b = to_y(b);
+            } else if (bnd) {
+                b.u = -a.u;
+            } else {
+                // the high-side face with the low-side face's normal discharge
+                const int k = vert ? r : c, ge = vert ? x0 + e : P.j0 + y0 + e;
+                const double qn = -*seam_slot(vert, 0, k, ge), qt = *seam_slot(vert, 1, k, ge);
+                velocity(b.h, vert ? qn : qt, vert ? qt : qn, b.u, b.v);
+                if (!vert) b = to_y(b);
             }
-            return;
         }
+        if (P.dry_skip && a.h == 0.0 && b.h == 0.0) {
+            // Both faces dry (h == 0 exactly, which also excludes NaN): every
+            // velocity, flux and depth is a zero, the hydrostatic depths are
+            // max(-H + min(H_a, H_b), 0) = 0, both wave speeds are 0, so all
+            // ten fluctuations evaluate to zeros.  They are stored as +0 (the
+            // full evaluation can give -0 for some; a zero's sign does not
+            // reach any non-zero value of this scheme).  Dry land makes this
+            // the common edge of a coastal grid.
+#pragma unroll
+            for (int f = 0; f < 5; f++) {
+                if (outM) outM[f * FS] = 0.0;
+                if (outP) outP[f * FS] = 0.0;
+            }
+            continue;
+        }
+        if (n < 0) {  // the grid's west and south edges: the normal points out of the grid
+            a.u = -a.u;
+            a.v = -a.v;
+            b.u = -b.u;
+            b.v = -b.v;
+        }
+        if (!put_edge<true>(P, a, b, fixed, outM, outP, FS)) put_edge_any(P, a, b, fixed, outM, outP, FS);
+        if (n < 0) {
+            outM[FS] = -outM[FS];
+            outM[2 * FS] = -outM[2 * FS];
+        }
+    }
+    bool own_ok = true;
+    if (own_tma) own_ok = mbar_wait_first(&sBarOwn, 0);  // the owned cells' U^n and extrema (bounded wait)
+    if (__syncthreads_or(!own_ok)) {
+        if (tid == 0) {
+            A.scal[SC_ERR] = 1.0;
+            mbar_wait(&sBarOwn, 0);
+        }
+        return;
     }
 
     // ---- phase 5: cell update
@@ -566,33 +759,22 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
             vk[1] -= dtax * kG * vc[0] * sDeta[ty * TX + tx];
             vk[2] -= dtay * kG * vc[0] * sDeta[TY * TX + ty * TX + tx];
         }
-        // friction (GPU/Reconstructor.cu:33-55) and erosion/deposition
-        // (:57-88) from U^n; one velocity evaluation serves both.
-        {
-            double ux, uy;
-            velocity(v0[0], v0[1], v0[2], ux, uy);
-            double modu = dsqrt(ux * ux + uy * uy);
-            if (P.manning) {  // GPU/Reconstructor.cu:47-50 as written (multiplies)
-                const double cm = dt * P.FR * P.FR * modu / pow(v0[0], 4.0 / 3.0);
-                vk[1] *= cm;
-                vk[2] *= cm;
-            } else {
-                double cf = ddiv(dt * P.FR * modu, v0[0] + kEpsilon);
-                vk[1] = ddiv(vk[1], 1.0 + cf);
-                vk[2] = ddiv(vk[2], 1.0 + cf);
+        {  // friction and erosion/deposition from U^n
+            double k1 = vk[1], k2 = vk[2], phi;
+            if (P.manning || !wet_divisor(v0[0]) || !sources<true>(P, dt, v0, k1, k2, phi)) {
+                State5 v;
+                v.h = v0[0];
+                v.qx = v0[1];
+                v.qy = v0[2];
+                v.H = v0[3];
+                v.hc = v0[4];
+                const Sources r = sources_any(P, dt, v, vk[1], vk[2]);
+                k1 = r.k1;
+                k2 = r.k2;
+                phi = r.phi;
             }
-            double c = ddiv(v0[4], v0[0] + P.eps_h);
-            double Z = ddiv(P.k.A_er * (modu * P.k.sqrt_FR), P.k.vs);
-            double Z5 = Z * Z * Z * Z * Z;
-            double Es = ddiv(1.3e-7 * Z5, 1 + 4.3e-7 * Z5);
-            double Fe = P.k.VP * Es;
-            if (Fe > 0.1) Fe = 0.1;
-            Fe = Fe * (double)(Fe > 0.0);
-            double Cb = P.k.K_dep * c;
-            double Fd = P.k.vs * Cb;
-            if (Fd > 0.1) Fd = 0.1;
-            Fd = Fd * (double)(Fd > 0.0);
-            double phi = (Fe - Fd) * (double)P.suspension;
+            vk[1] = k1;
+            vk[2] = k2;
             vk[3] -= dt * phi;
             vk[4] += dt * phi;
         }
@@ -601,7 +783,13 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
 #pragma unroll
         for (int f = 0; f < 5; f++) {
             double FL = sFlux[(0 * 5 + f) * FS + cell], FR = sFlux[(1 * 5 + f) * FS + cell];
-            double FD = sFlux[(2 * 5 + f) * FS + cell], FU = sFlux[(3 * 5 + f) * FS + cell];
+            // y fluctuations back to x/y components (GPU/VolumeSolver.cu:129-152)
+            const int fy = (f == 1) ? 2 : (f == 2) ? 1 : f;
+            double FD = sFlux[(2 * 5 + fy) * FS + cell], FU = sFlux[(3 * 5 + fy) * FS + cell];
+            if (f == 1) {
+                FD = -FD;
+                FU = -FU;
+            }
             vk[f] -= invx * (FL + FR) + invy * (FD + FU);
         }
         // RK combine + filter, GPU/Volume_kernel.cu:244-281; MUSCL-Hancock
@@ -625,7 +813,27 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
             z = coef0 * v0[3] + coef1 * vk[3];
             hc = coef0 * v0[4] + coef1 * vk[4];
         }
-        positivity_filter(h, qx, qy, hc);
+        double d;  // last stage: the new cell's CFL step
+        {
+            bool ok = wet_divisor(h);
+            double fh = h, fx = qx, fy = qy, fc = hc;
+            if (ok) {
+                const Face5 f = filter_face<true>(fh, fx, fy, z, fc, ok);
+                if (LAST) ok &= cfl_dt_fast(P, f, d);
+            }
+            if (!ok) {
+                fh = h;
+                fx = qx;
+                fy = qy;
+                fc = hc;
+                positivity_filter(fh, fx, fy, fc);
+                if (LAST) d = cfl_dt(P, fh, fx, fy);
+            }
+            h = fh;
+            qx = fx;
+            qy = fy;
+            hc = fc;
+        }
         Vout[gown] = h;
         Vout[plane + gown] = qx;
         Vout[2 * plane + gown] = qy;
@@ -642,7 +850,6 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
                 A.bmin[gown] = fmax(A.bmin[gown], z);
                 if (h > eps_h) A.eta_max[gown] = fmax(A.eta_max[gown], h - z);
             }
-            double d = cfl_dt(P, h, qx, qy);
             if (!isnan(d)) dtcell = d;
             bad = !(finite64(h) && finite64(qx) && finite64(qy) && finite64(z) && finite64(hc));
         }
@@ -793,6 +1000,10 @@ EncodeTiledFn tensor_map_encoder() {
 
 namespace {
 
+// At most one wave of 32 x 8 tiles (two CTAs on each of 148 SMs): 16 x 4 tiles
+// instead.  48 x 36 cells, 64 steps: 32 x 8 tiles 1017 us, 16 x 4 615 us.
+constexpr long long kSmallTiles = 296;
+
 struct Variant {
     int tx, ty, nthr, own;
     size_t smem;
@@ -816,37 +1027,34 @@ Variant make_variant() {
     return v;
 }
 
-const Variant &variant() {
-    static Variant v = [] {
+// The variant of a grid of npx x npy (owned) cells; every one gives the same
+// values.
+const Variant &variant(int npx, int npy) {
+    static const bool fixed = std::getenv("TSU_TILE64") != nullptr;
+    static const Variant v = [] {
         const char *e = std::getenv("TSU_TILE64");
         if (e && !std::strcmp(e, "16x16")) return make_variant<16, 16, 2>();
-        if (e && !std::strcmp(e, "32x16")) return make_variant<32, 16, 1>();
-        if (e && !std::strcmp(e, "16x8")) return make_variant<16, 8, 4>();
-        if (e && !std::strcmp(e, "32x4")) return make_variant<32, 4, 4>();
+        if (e && !std::strcmp(e, "16x4")) return make_variant<16, 4, 3, 192, 2>();
         if (e && !std::strcmp(e, "32x8t256")) return make_variant<32, 8, 2, 256>();
-        if (e && !std::strcmp(e, "32x8t288")) return make_variant<32, 8, 2, 288>();
-        if (e && !std::strcmp(e, "32x8t352")) return make_variant<32, 8, 2, 352>();
-        if (e && !std::strcmp(e, "32x8t384")) return make_variant<32, 8, 2, 384>();
         if (e && !std::strcmp(e, "32x8t320reg")) return make_variant<32, 8, 2, 320, 0>();
         if (e && !std::strcmp(e, "32x8t320late")) return make_variant<32, 8, 2, 320, 1>();
         // default: 32 x 8 tile, 320 threads, 2 CTAs per SM (shared memory
-        // allows 2; 20 warps per SM at 92-96 registers, no spills), the
-        // second stage's U^n and extrema staged by TMA (OWN = 2, 107 KB of
-        // shared memory per CTA).  Measured at 4096^2: 256 threads 2161, 288
-        // 2308, 320 2514, 352 2365, 384 2331 Mcell-steps/s; with 320 threads
-        // OWN = 0 / 1 / 2: 2533 / 2566 / 2585 (one box, 100 steps).  Every
-        // choice is value-identical.
+        // allows 2; 20 warps per SM at 96 registers), the second stage's U^n
+        // and extrema staged by TMA (OWN = 2, 111 KB of shared memory per CTA).
         return make_variant<32, 8, 2, 320, 2>();
     }();
-    return v;
+    // Small grids: 16 x 4 tiles of 192 threads.  Every phase of a tile is then
+    // one round of its six warps (the 32 x 8 tile needs two of its ten), and
+    // four times as many SMs have work.
+    static const Variant small = make_variant<16, 4, 3, 192, 2>();
+    const long long tiles = (long long)((npx + 31) / 32) * ((npy + 7) / 8);
+    return (!fixed && tiles <= kSmallTiles) ? small : v;
 }
 
 }  // namespace
 
-size_t stage64_smem_bytes() { return variant().smem; }
-
-cudaError_t stage64_prepare() {
-    const Variant &v = variant();
+cudaError_t stage64_prepare(int npx, int npy) {
+    const Variant &v = variant(npx, npy);
     for (int i = 0; i < 5; i++) {
         cudaError_t e = cudaFuncSetAttribute(v.k[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v.smem);
         if (e != cudaSuccess) return e;
@@ -856,9 +1064,9 @@ cudaError_t stage64_prepare() {
 
 bool stage64_tma_maps(const double *bufA, const double *bufB, const unsigned char *mask, const double *const ext[3],
                       long long pitch, long long plane, int npx, int npy, CUtensorMap *tmA, CUtensorMap *tmB,
-                      CUtensorMap *tmM, CUtensorMap *tmO, CUtensorMap tmE[3]) {
+                      CUtensorMap *tmM, CUtensorMap *tmO, CUtensorMap tmE[3], int rows) {
     EncodeTiledFn f = tensor_map_encoder();
-    const Variant &v = variant();
+    const Variant &v = variant(npx, rows);
     if (!f || npx < v.tx + 4 || npy < v.ty + 4) return false;
     if (reinterpret_cast<uintptr_t>(bufA) % 16 || reinterpret_cast<uintptr_t>(bufB) % 16 ||
         reinterpret_cast<uintptr_t>(mask) % 16 || pitch % 16)
@@ -897,12 +1105,12 @@ bool stage64_tma_maps(const double *bufA, const double *bufB, const unsigned cha
 }
 
 dim3 stage64_grid(int npx, int npy) {
-    const Variant &v = variant();
+    const Variant &v = variant(npx, npy);
     return dim3((npx + v.tx - 1) / v.tx, (npy + v.ty - 1) / v.ty);
 }
 
 cudaError_t stage64_launch(int order, int stage, const Stage64Args &a, cudaStream_t st) {
-    const Variant &v = variant();
+    const Variant &v = variant(a.phys.npx, a.phys.npy);
     dim3 g = stage64_grid(a.phys.npx, a.phys.npy);
     int which = (order == 2) ? (stage == 0 ? 0 : 1) : 2;
     if (a.phys.rk == 0) which = (order == 2) ? 3 : 4;  // MUSCL-Hancock: one stage

@@ -72,8 +72,7 @@ __device__ __forceinline__ double finalize_dt(double m, long long ncells) {
     return m;
 }
 
-size_t stage64_smem_bytes();
-cudaError_t stage64_prepare();
+cudaError_t stage64_prepare(int npx, int npy);
 dim3 stage64_grid(int npx, int npy);
 cudaError_t stage64_launch(int order, int stage, const Stage64Args &a, cudaStream_t st);
 cudaError_t initial_dt_launch(const double *V, long long pitch, long long plane, const Phys64 &P, double *partials,
@@ -92,9 +91,9 @@ constexpr unsigned long long kDefaultWaitNs = 500000000ull;  // async.cuh kWaitN
 // tile shape; false if the driver cannot (the kernels then load with
 // ordinary instructions)
 // (tmO, tmE[3]: the owned-cell boxes of bufA and of the extrema hmax, bmin,
-// eta_max)
+// eta_max; npy: the stored rows, rows: the owned ones)
 bool stage64_tma_maps(const double *bufA, const double *bufB, const unsigned char *mask, const double *const ext[3],
                       long long pitch, long long plane, int npx, int npy, CUtensorMap *tmA, CUtensorMap *tmB,
-                      CUtensorMap *tmM, CUtensorMap *tmO, CUtensorMap tmE[3]);
+                      CUtensorMap *tmM, CUtensorMap *tmO, CUtensorMap tmE[3], int rows);
 
 }  // namespace tsu
