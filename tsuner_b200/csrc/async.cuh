@@ -67,8 +67,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity) {
 // waits run out while the copies are still in flight; the drain waits above
 // keep the full limit, so a CTA never leaves with its own copies or MMAs
 // still running.  One copy per compilation unit (set through that unit's
-// set_wait_limit_* host function on the current device).
-static __device__ unsigned long long g_wait_limit_ns = kWaitNs;
+// set_wait_limit_* host function on the current device).  Constant memory: a
+// wait reads it without a round trip to L2.
+static __constant__ unsigned long long g_wait_limit_ns = kWaitNs;
 // non-blocking probe of the phase (try_wait may suspend the thread until the
 // phase completes, for a hardware-chosen time)
 __device__ __forceinline__ bool mbar_test(uint64_t *bar, unsigned parity) {
@@ -83,8 +84,16 @@ __device__ __forceinline__ bool mbar_test(uint64_t *bar, unsigned parity) {
     return ok != 0;
 }
 __device__ __forceinline__ bool mbar_wait_first(uint64_t *bar, unsigned parity) {
-    const unsigned long long lim = *static_cast<volatile unsigned long long *>(&g_wait_limit_ns);
-    if (lim >= kWaitNs) return mbar_wait_for(bar, parity, lim);
+    if (mbar_test(bar, parity)) return true;  // the usual case in a pipeline: no clock is read
+    const unsigned long long lim = g_wait_limit_ns;
+    if (lim >= kWaitNs) {
+        // try_wait suspends the thread for a while by itself; the global timer
+        // takes far longer to read than an ordinary wait lasts
+#pragma unroll 1
+        for (int i = 0; i < 32; i++)
+            if (mbar_try(bar, parity)) return true;
+        return mbar_wait_for(bar, parity, lim);
+    }
     // a lowered limit (tests of the error path): poll without suspending, so
     // that the limit, not try_wait's own suspension, decides
     const unsigned long long t0 = gtimer();

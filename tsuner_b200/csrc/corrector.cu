@@ -11,34 +11,24 @@
 // Y[y][x] = sum W[tap] X[y+dy][x+dx], zero padding); FP32 master weights,
 // bias and Adam moments.
 //
+// Both convolution kernels read their shifted operands in place: a tile of
+// pixels lies in shared memory as TMA writes it, one pixel's 32 channels per
+// 64-byte row with the 64-byte swizzle, and an MMA operand is a start address
+// and two strides into it (sdesc64).
+//
 // Forward / input-gradient convolution (conv3x3_fwd_kernel): implicit GEMM
-//   D[128 pixels x 32 cout] = sum over 9 taps x 2 channel halves of
-//   A_tap,h[128 x 16] . B_tap,h[16 x 32]  (18 MMAs of M=128, N=32, K=16)
-// over an 8 x 16 pixel tile.  The input patch (10 x 18 pixels with the halo)
-// is stored in shared memory as four channel-quarter planes (16 bytes per
-// pixel per plane), which makes every A_tap,h a K-major no-swizzle operand
-// that starts inside the patch: core matrix = 8 consecutive pixels of one
-// tile row (16-byte rows), the two K chunks one plane apart (LBO = plane
-// size) and the 16 row groups one patch row apart (SBO = 160 B).  No im2col
-// copy is made.  The patch arrives by TMA: four 4-D box loads per tile (one
-// per channel quarter, zero fill outside the image = the convolution's
-// padding) completing on an mbarrier.  CTAs are persistent; the patch and the
-// TMEM accumulator are double-buffered so that the load of tile i+1 and the
-// epilogue of tile i-1 overlap the MMAs of tile i.
+// whose M = 128 rows are 16 groups of 8 pixels of one image row each and whose
+// N = 96 columns are the contributions of an input row to the three output
+// rows around it, 6 MMAs (3 column offsets x 2 channel halves, K = 16) per
+// input row.  8 x 528^2 pixels, BF16 with ReLU: 105 -> 69 us from HBM (the 285
+// MB it reads and writes take 44 us), 98 -> 57 us when the input is in L2.
 //
 // Weight gradient (conv3x3_wgrad_kernel): dW[cout][tap][cin] =
 //   sum_p dZ[p][cout] X[p + off(tap)][cin], a GEMM with the pixels as the
-// reduction dimension.  The input patch is loaded by one TMA box of a 5-D
-// view of the NHWC tensor that lands as [row][channel quarter][x][8
-// channels]: for a horizontal tap offset dx, the 12 core-matrix groups
-// (dy, quarter) of the shifted patch are then 160 B apart, so
-// D_dx[dy * 32 + cin][cout] is one M = 128 MMA per 16 pixels with A read in
-// place (rows 96..127 see the next patch row and are ignored) and B = the dZ
-// tile as loaded; no operand copy is made.  Three accumulators (dx = 0..2)
-// take 96 TMEM columns.  Two stages: the next tile loads while this one's
-// MMAs run.  The bias gradient is summed from the dZ tile on the CUDA cores.
-// Each CTA accumulates a strip of tiles in TMEM and adds its partial result
-// to the FP32 gradients with atomics.
+// reduction dimension; all nine taps in one MMA per 16 pixels (M = the three
+// row offsets x cin, N = the three column offsets x cout).  8 x 528^2: kernel
+// 100 -> 50 us, the call with its reduction 185 -> 75 us.  The bias gradient
+// is summed from the dZ tile on the CUDA cores.
 //
 // Every mbarrier wait is bounded (globaltimer); on expiry the kernel sets
 // the error word, waits once more (bounded) for its MMAs, frees its TMEM and
@@ -52,6 +42,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <vector>
 
@@ -64,46 +55,47 @@ namespace corr {
 
 typedef __nv_bfloat16 bf16;
 
-constexpr int C = 32;                       // channels
-constexpr int TXP = 8, TYP = 16;            // output tile (128 pixels)
-constexpr int PW = TXP + 2, PH = TYP + 2;   // patch 10 x 18
-constexpr int PPIX = PW * PH;               // 180
-constexpr int kPlaneData = PPIX * 16;       // one channel-quarter plane: 2880 B
-constexpr int kPlane = 2944;                // plane stride: 23 x 128 B (TMA destinations 128-byte aligned)
-constexpr int kPatch = 4 * kPlane;          // 11776 B
-constexpr int kWBytes = 9 * 4 * 32 * 16;    // weights: 18432 B
-constexpr int KROWS = 9 * C;                // 288
+constexpr int C = 32;        // channels
+constexpr int kPix = C * 2;  // one pixel: 64 B, the span of the 64-byte swizzle
+constexpr int KROWS = 9 * C; // 288
 
-// patch buffers: tile i+1 loads while tile i's MMAs run and tile i-1's
-// epilogue stages its output in the buffer tile i-1 was read from
-constexpr int kFwdBufs = 3;
-constexpr int kFwdSmem = 1024 + kWBytes + kFwdBufs * kPatch + 64;
-constexpr int kFwdCtasPerSm = 4;  // 4 x (54 KB + 1 KB) of shared memory, 4 x 64 TMEM columns
-static_assert(kFwdCtasPerSm * (kFwdSmem + 1024) <= 228 * 1024 && kFwdCtasPerSm * 64 <= 512, "fwd residency");
-static_assert(kPlane % 128 == 0 && kPlane >= kPlaneData && kWBytes % 128 == 0, "TMA destinations");
-// warp-specialised forward (conv3x3_fwd_ws_kernel): warp 0 loads patches,
-// warp 1 issues the MMAs, warps 2-5 run the epilogue.  A ring of kWsBufs
-// patch buffers (full / empty barriers) and kWsAcc TMEM accumulators of 32
-// columns (full / empty barriers); the epilogue stages its output in a 2 KB
-// area per warp of its own.
-constexpr int kWsBufs = 6, kWsAcc = 4, kWsThreads = 192;
-constexpr int kWsStage = 4 * 2048;
-constexpr int kWsBarBytes = (2 * kWsBufs + 2 * kWsAcc) * 8 + 32;
-constexpr int kWsSmem = 1024 + kWBytes + kWsBufs * kPatch + kWsStage + kWsBarBytes;
-constexpr int kWsCtasPerSm = 2;  // 2 x (~98 KB + 1 KB) of shared memory, 2 x 128 TMEM columns
-static_assert(kWsCtasPerSm * (kWsSmem + 1024) <= 228 * 1024 && kWsCtasPerSm * 32 * kWsAcc <= 512, "ws residency");
-// wgrad: patch + dZ tile + A for half of the 8 K steps (4 x 3 M blocks x 4 KB);
-// ~67 KB, so three CTAs fit on an SM
-constexpr int kZPlane = 128 * 16;
-// weight gradient: the patch as [row][channel quarter][x][8 channels]
-constexpr int kRowQ = 4 * PW * 16;           // one patch row: 640 B
-constexpr int kWgPatch = PH * kRowQ;         // 11520 B
-constexpr int kWgPatchBuf = 12288;           // + the row read by the ignored A rows 96..127
-constexpr int kWgStage = kWgPatchBuf + 4 * kZPlane;
-constexpr int kWgSmem = 1024 + 2 * kWgStage + 64;
-constexpr int kWgCtasPerSm = 4;              // 128 TMEM columns each
-static_assert(kWgPatch + kRowQ <= kWgPatchBuf && kWgPatchBuf % 128 == 0 && kWgStage % 128 == 0, "wgrad buffers");
-static_assert(kWgCtasPerSm * (kWgSmem + 1024) <= 228 * 1024 && kWgCtasPerSm * 128 <= 512, "wgrad residency");
+// forward (conv3x3_fwd_kernel)
+constexpr int GX = 8, NG = 16;               // columns of a group, groups of a tile row (M = 128 pixels)
+constexpr int GW = GX + 2;                   // columns loaded per group
+constexpr int kCRows = 4;                    // input rows per chunk
+constexpr int kGRow = GW * kPix;             // one group's row: 640 B
+constexpr int kGrpBytes = kCRows * kGRow;    // 2560 B
+constexpr int kChunk = NG * kGrpBytes;       // 40960 B
+constexpr int kChunks = 2;                   // chunk ring
+constexpr int kWBytes = 9 * 4 * 32 * 16;     // weights: 18432 B
+constexpr int kWBlk = 96 * 16;               // one (dx, channel quarter): 3 dy x 32 cout rows of 16 B
+constexpr int kAcc = 8;                      // TMEM accumulators (output rows) of 32 columns
+constexpr int kEpiWarps = 4;
+constexpr int kFwdCtas = 2;                  // CTAs per SM: one's issuing covers the other's
+constexpr int kFwdThreads = 64 + 32 * kEpiWarps;
+constexpr int kStage = kEpiWarps * 2048;
+constexpr int kFwdBars = (2 * kChunks + 2 * kAcc + 1) * 8 + 32;
+constexpr int kFwdSmem = 1024 + kWBytes + kChunks * kChunk + kStage + kFwdBars;
+static_assert(kGrpBytes % 512 == 0 && kWBytes % 512 == 0, "swizzled TMA destinations");
+static_assert(kFwdCtas * (kFwdSmem + 1024) <= 228 * 1024 && kFwdCtas * 32 * kAcc <= 512, "residency");
+
+// weight gradient (conv3x3_wgrad_kernel)
+constexpr int TYP = 16;                          // tile: 8 columns x 16 rows (K = 128 pixels)
+constexpr int kXRow = GX * kPix;                 // 512 B
+constexpr int kXBytes = (TYP + 2) * kXRow;       // 9216 B loaded
+constexpr int kXBuf = (TYP + 3) * kXRow;         // + the row read by the ignored rows 96..127 of A
+constexpr int kZBytes = TYP * kGRow;             // 10240 B
+constexpr int kWgStage = kXBuf + kZBytes;        // 19968 B
+constexpr int kWgStages = 8;
+constexpr int kWgThreads = 192;
+// tiles summed in TMEM before the sum moves to registers: the tensor cores add
+// to an FP32 accumulator with truncation, whose bias grows with the number of
+// additions (8 x 528^2: relative error of dW against 64 bits 1.4e-5 with all
+// 118 tiles of a CTA in one accumulator, 3e-6 with at most 30)
+constexpr int kWgFlush = 24;
+constexpr int kWgSmem = 1024 + kWgStages * kWgStage + (2 * kWgStages + 5) * 8 + 32;
+static_assert(kXBuf % 512 == 0 && kWgStage % 512 == 0, "swizzled TMA destinations");
+static_assert(kWgSmem + 1024 <= 228 * 1024, "one CTA per SM");
 
 __device__ int g_corr_err;  // set by a kernel whose wait expired
 
@@ -111,6 +103,17 @@ __device__ int g_corr_err;  // set by a kernel whose wait expired
 __device__ __forceinline__ uint64_t sdesc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
     return (uint64_t)((addr >> 4) & 0x3FFF) | ((uint64_t)((lbo >> 4) & 0x3FFF) << 16) |
            ((uint64_t)((sbo >> 4) & 0x3FFF) << 32) | ((uint64_t)1 << 46);
+}
+
+// the same with the 64-byte swizzle.  K-major operands: rows of 64 B, sbo = the
+// stride of 8-row groups (lbo unused).  MN-major operands: lbo = the stride of
+// 32-element blocks along M or N, sbo = the stride of 8-row groups along K.
+// The hardware swizzles the final shared-memory address (16-byte chunk index
+// ^= address bits 7-8), as TMA does when it writes, so an operand may start
+// at any pixel of a tile and its blocks may overlap: a convolution's shifted
+// operands are start addresses and strides into one tile.
+__device__ __forceinline__ uint64_t sdesc64(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+    return sdesc(addr, lbo, sbo) | ((uint64_t)4 << 61);
 }
 
 // kind::f16 instruction descriptor: D FP32, A/B BF16, majors, N, M
@@ -144,6 +147,14 @@ __device__ __forceinline__ void mma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
 }
+// true in one lane of a converged warp.  A role's loop runs in the whole warp,
+// so that its counters and descriptors stay in uniform registers, which the
+// MMA takes its operands from; only the issuing itself is one lane's.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -176,26 +187,19 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
     return *reinterpret_cast<uint32_t *>(&h);
 }
 
-struct TileGeom {
-    int ntx, nty, per_img, total;
+// The forward kernel's work: the images' columns in groups of 8, 16 groups to
+// a set (one tile row of a set is M = 128 pixels, of any images), and the sets'
+// rows, numbered set by set, shared out evenly among the CTAs.
+struct FwdGeom {
+    int ntx, groups, sets, rows;  // groups per image row, groups in all, sets, rows of all sets
 };
-__host__ __device__ inline TileGeom tile_geom(int nimg, int H, int W) {
-    TileGeom g;
-    g.ntx = (W + TXP - 1) / TXP;
-    g.nty = (H + TYP - 1) / TYP;
-    g.per_img = g.ntx * g.nty;
-    g.total = nimg * g.per_img;
+__host__ __device__ inline FwdGeom fwd_geom(int nimg, int H, int W) {
+    FwdGeom g;
+    g.ntx = (W + GX - 1) / GX;
+    g.groups = nimg * g.ntx;
+    g.sets = (g.groups + NG - 1) / NG;
+    g.rows = g.sets * H;
     return g;
-}
-
-// 10 x 18 x 32 input patch (zero fill outside the image) -> four
-// channel-quarter planes: one TMA box (8 channels x 10 x 18) per plane.  The
-// innermost coordinate (channel 8q) is a multiple of 16 bytes; the halo may
-// start at x0 - 1 = -1 or y0 - 1 = -1, which loads zeros.
-__device__ __forceinline__ void issue_patch(const CUtensorMap *map, int img, int x0, int y0, unsigned char *patch,
-                                            uint64_t *bar) {
-#pragma unroll
-    for (int q = 0; q < 4; q++) tma_load_4d(patch + q * kPlane, map, 8 * q, x0 - 1, y0 - 1, img, bar);
 }
 
 struct ConvArgs {
@@ -210,49 +214,60 @@ struct ConvArgs {
     float *Y2;           // FP32 output of channels 0 and 1 only, [pixel][2] (the corrector's last layer)
 };
 
-// Epilogue of one tile: TMEM accumulators (lane = pixel, column = output
-// channel) + bias, ReLU, optional gate, then the store.  A warp holds 32
-// pixels = 4 tile rows of 8; in NHWC each tile row is one contiguous run of
-// 8 x 32 channels.  BF16 output (every layer but the last, and the input
-// gradients) goes through `stage` (2 KB per warp, the patch buffer the tile's
-// MMAs have finished reading): each lane writes its pixel's 4 x 16 B, then
-// each instruction stores one tile row as 32 lanes x 16 B contiguous.
-// 16-byte chunk k of pixel p sits in slot p * 4 + (k ^ ((p >> 1) & 3)), so
-// both patterns are free of bank conflicts.  FP32 output (the last layer)
-// goes the same way in two halves of 16 channels.  The gate is read per
-// pixel (staging it too measured slower: 131 vs 110 us per 8 x 512^2 launch).
-__device__ __forceinline__ void conv_epilogue(const ConvArgs &a, const TileGeom &G, int t, uint32_t taddr, int warp,
-                                              int lane, const float *sBias, unsigned char *stage,
-                                              uint64_t *release = nullptr) {
-    const int img = t / G.per_img, r = t - img * G.per_img;
-    const int tyi = r / G.ntx, txi = r - tyi * G.ntx;
-    const int x0 = txi * TXP, y0 = tyi * TYP;
-    // this lane's pixel (TMEM lane = pixel: 8 per tile row, 4 rows per warp)
-    const int gx = x0 + (lane & 7), gy = y0 + warp * 4 + (lane >> 3);
-    const bool inside = gx < a.W && gy < a.H;
-    const long long o = inside ? (((long long)img * a.H + gy) * a.W + gx) * C : 0;
+// A CTA's run of rows [b, e) of FwdGeom::rows, one segment (a range of rows of
+// one set) at a time.
+struct Segments {
+    int H, at, end, set, y0, y1;
+    __device__ __forceinline__ Segments(int H_, int rows, int cta, int nctas) : H(H_) {
+        at = (int)((long long)rows * cta / nctas);
+        end = (int)((long long)rows * (cta + 1) / nctas);
+        set = y0 = y1 = 0;
+    }
+    __device__ __forceinline__ bool next() {
+        if (at >= end) return false;
+        set = at / H;
+        y0 = at - set * H;
+        y1 = min(H, y0 + (end - at));
+        at += y1 - y0;
+        return true;
+    }
+};
+
+// Epilogue of 32 pixels (4 groups of 8) of output row y: TMEM accumulators
+// (lane = pixel, column = output channel) + bias, ReLU, optional gate, then
+// the store.  In NHWC a group's row is one contiguous run of 8 x 32 channels.
+// BF16 output (every layer but the last, and the input gradients) goes through
+// `sw` (2 KB of this warp): each lane writes its pixel's 4 x 16 B, then each
+// instruction stores one group's row as 32 lanes x 16 B contiguous.  16-byte
+// chunk k of pixel p sits in slot p * 4 + (k ^ ((p >> 1) & 3)), so both
+// patterns are free of bank conflicts.  FP32 output goes the same way in two
+// halves of 16 channels.  The gate is read per pixel.
+// px: element offset of this lane's own pixel at row 0 (-1: outside), row[r]:
+// of the pixel and chunk this lane stores of group r (-1: outside).
+__device__ __forceinline__ void conv_epilogue(const ConvArgs &a, int y, uint32_t taddr, int lane, const float *sBias,
+                                              uint4 *sw, const long long px, const long long (&row)[4],
+                                              uint64_t *release) {
+    const long long yo = (long long)y * a.W * C;
     // the gate (4 x 16 B of this pixel; the lines stay in L1 across the 4
     // loads) is requested before the TMEM read so the two latencies overlap
     uint4 g[4];
-    if (a.gate && inside) {
-        const uint4 *gp = reinterpret_cast<const uint4 *>(a.gate + o);
+    if (a.gate && px >= 0) {
+        const uint4 *gp = reinterpret_cast<const uint4 *>(a.gate + px + yo);
 #pragma unroll
         for (int k = 0; k < 4; k++) g[k] = __ldg(gp + k);
     }
     float acc[32];
-    tmem_ld32(taddr + ((uint32_t)(warp * 32) << 16), acc);
-    if (release) {  // the accumulator is in registers: hand its TMEM columns back to the MMA issuer
-        fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(release);
-    }
+    tmem_ld32(taddr, acc);
+    fence_before();  // the accumulator is in registers: hand its TMEM columns back to the MMA issuer
+    __syncwarp();
+    if (lane == 0) mbar_arrive(release);
 #pragma unroll
     for (int n = 0; n < 32; n++) {
         float v = acc[n] + sBias[n];
         if (a.relu) v = fmaxf(v, 0.f);
         acc[n] = v;
     }
-    if (a.gate && inside) {
+    if (a.gate && px >= 0) {
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const uint32_t w[4] = {g[k].x, g[k].y, g[k].z, g[k].w};
@@ -264,11 +279,10 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs &a, const TileGeom 
             }
         }
     }
-    uint4 *sw = reinterpret_cast<uint4 *>(stage + warp * 2048);
-    const int rx = lane >> 2, kc = lane & 3;  // row phase: pixel in the tile row, 16-byte chunk
+    const int rx = lane >> 2, kc = lane & 3;  // row phase: pixel of the group, 16-byte chunk
     const int own = (lane >> 1) & 3;          // swizzle of this lane's own pixel
-    if (a.Y2) {  // the two used channels: 8 B per pixel, a tile row is 64 contiguous bytes
-        if (inside) *reinterpret_cast<float2 *>(a.Y2 + (o / C) * 2) = make_float2(acc[0], acc[1]);
+    if (a.Y2) {  // the two used channels: 8 B per pixel, a group's row is 64 contiguous bytes
+        if (px >= 0) *reinterpret_cast<float2 *>(a.Y2 + (px + yo) / C * 2) = make_float2(acc[0], acc[1]);
         return;
     }
     if (a.Yf) {  // FP32: two halves of 16 channels (64 B per pixel) through the same 2 KB
@@ -283,18 +297,14 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs &a, const TileGeom 
             __syncwarp();
             uint4 v[4];
 #pragma unroll
-            for (int rr = 0; rr < 4; rr++) {
-                const int p = rr * 8 + rx;
-                v[rr] = sw[p * 4 + (kc ^ ((p >> 1) & 3))];
+            for (int r = 0; r < 4; r++) {
+                const int p = r * 8 + rx;
+                v[r] = sw[p * 4 + (kc ^ ((p >> 1) & 3))];
             }
             __syncwarp();  // the next half overwrites the slots
 #pragma unroll
-            for (int rr = 0; rr < 4; rr++) {
-                const int ox = x0 + rx, oy = y0 + warp * 4 + rr;
-                if (ox < a.W && oy < a.H)
-                    *reinterpret_cast<uint4 *>(a.Yf + (((long long)img * a.H + oy) * a.W + ox) * C + 16 * hf +
-                                               kc * 4) = v[rr];
-            }
+            for (int r = 0; r < 4; r++)  // row[] counts 8 channels a chunk; here a chunk is 4
+                if (row[r] >= 0) *reinterpret_cast<uint4 *>(a.Yf + row[r] - kc * 4 + 16 * hf + yo) = v[r];
         }
         return;
     }
@@ -305,176 +315,72 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs &a, const TileGeom 
     __syncwarp();
     uint4 v[4];  // all four rows read before the first global store
 #pragma unroll
-    for (int rr = 0; rr < 4; rr++) {
-        const int p = rr * 8 + rx;
-        v[rr] = sw[p * 4 + (kc ^ ((p >> 1) & 3))];
+    for (int r = 0; r < 4; r++) {
+        const int p = r * 8 + rx;
+        v[r] = sw[p * 4 + (kc ^ ((p >> 1) & 3))];
     }
+    __syncwarp();  // the next row overwrites the slots
 #pragma unroll
-    for (int rr = 0; rr < 4; rr++) {
-        const int ox = x0 + rx, oy = y0 + warp * 4 + rr;
-        if (ox < a.W && oy < a.H)
-            *reinterpret_cast<uint4 *>(a.Ybf + (((long long)img * a.H + oy) * a.W + ox) * C + kc * 8) = v[rr];
-    }
+    for (int r = 0; r < 4; r++)
+        if (row[r] >= 0) *reinterpret_cast<uint4 *>(a.Ybf + row[r] + yo) = v[r];
 }
 
-__global__ void __launch_bounds__(128) conv3x3_fwd_kernel(ConvArgs a, const __grid_constant__ CUtensorMap tmX) {
+// Forward convolution.  Persistent, two CTAs per SM; a CTA's rows come in
+// segments.
+//   warp 0: input rows of the segment, kCRows at a time: lane i loads group i's
+//     box (10 columns x 4 rows x 32 channels) into the chunk ring;
+//   warp 1 (lane 0): for each input row r, the MMAs A_dx,h[128 x 16] .
+//     B_dx,h[16 x 96] of the 3 column offsets and 2 channel halves: N = 96 are
+//     the contributions to output rows r - 1, r, r + 1, whose accumulators are
+//     neighbours in a ring of kAcc TMEM column blocks.  An output row thus
+//     collects its taps in the order (dy, dx, half).  The first MMA of a row's
+//     first input overwrites (N = 32 of its own); at a segment's ends and
+//     where the ring wraps N is 32 or 64;
+//   warps 2-5: epilogue, a quarter of the row's pixels each.
+// What bounded the one-tap form (18 MMAs of N = 32 per 128 pixels, the patch
+// as four 16-byte channel planes): each MMA reads 4 KB of A for 131 kFLOP, and
+// TMA writes 16 bytes at a time.  Here 6-7 MMAs read A once for three taps,
+// and a TMA row is a pixel's 64 bytes.  No role waits at a CTA barrier inside
+// its loop.  Every wait is bounded; a role whose wait expires sets the error
+// word and leaves its loop, the others' waits then expire in turn, and before
+// TMEM is freed the issued MMAs and loads are waited for.
+__global__ void __launch_bounds__(kFwdThreads, kFwdCtas)
+    conv3x3_fwd_kernel(const __grid_constant__ ConvArgs a, const __grid_constant__ CUtensorMap tmX) {
     extern __shared__ unsigned char sm_raw[];
     unsigned char *sm = smem_align<1024>(sm_raw);
     unsigned char *sW = sm;
-    unsigned char *sP0 = sm + kWBytes;  // kFwdBufs patch buffers
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(sP0 + kFwdBufs * kPatch);  // [2] MMA done (per TMEM slot)
-    uint64_t *full = mbar + 2;                                               // [kFwdBufs] patch loaded
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(full + kFwdBufs);
-    static_assert((2 + kFwdBufs) * 8 + 4 <= 64, "barriers");
+    unsigned char *sP = sm + kWBytes;                  // chunk ring
+    unsigned char *sStage = sP + kChunks * kChunk;     // 2 KB per epilogue warp
+    uint64_t *full = reinterpret_cast<uint64_t *>(sStage + kStage);  // [kChunks] chunk landed
+    uint64_t *empty = full + kChunks;                                // [kChunks] chunk's MMAs done
+    uint64_t *accf = empty + kChunks;                                // [kAcc] accumulator ready
+    uint64_t *acce = accf + kAcc;                                    // [kAcc] accumulator read
+    uint64_t *fin = acce + kAcc;                                     // all MMAs done
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(fin + 1);
+    int *sCount = reinterpret_cast<int *>(tslot + 1);  // [0] chunks issued, [1] chunks waited for
     __shared__ float sBias[32];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const TileGeom G = tile_geom(a.nimg, a.H, a.W);
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const FwdGeom G = fwd_geom(a.nimg, a.H, a.W);
 
-    // weights -> [tap][quarter][cout] 16-byte rows (K-major B operand)
-    for (int c = tid; c < 32 * 36; c += 128) {
-        const int n = c / 36, r = c - n * 36;  // r = tap * 4 + quarter
-        cp_async16(sW + r * 512 + n * 16, a.Wk + n * KROWS + r * 8, 16);
+    // weights -> [dx][quarter][dy = +1, 0, -1][cout] rows of 16 B (K-major B operand, no swizzle)
+    for (int c = tid; c < 32 * 36; c += kFwdThreads) {
+        const int n = c / 36, r = c - n * 36, tap = r >> 2, q = r & 3;
+        const int dy = tap / 3, dx = tap - dy * 3;
+        cp_async16(sW + (dx * 4 + q) * kWBlk + ((2 - dy) * 32 + n) * 16, a.Wk + n * KROWS + r * 8, 16);
     }
     cp_async_commit();
     if (tid < 32) sBias[tid] = a.bias ? a.bias[tid] : 0.f;
-    if (warp == 0) tmem_alloc(tslot, 64);
+    if (warp == 1) tmem_alloc(tslot, 32 * kAcc);
     if (tid == 0) {
-        for (int k = 0; k < 2 + kFwdBufs; k++) mbar_init(&mbar[k], 1);
-        mbar_init_fence();
-    }
-    cp_async_wait_all();  // the weights
-    fence_async_smem();
-    fence_before();
-    __syncthreads();
-    fence_after();
-    const uint32_t tmem = *tslot;
-    const uint32_t id = idesc(128, 32, 0, 0);
-    const uint32_t w_u32 = smem_u32(sW);
-
-    // tile t of iteration k -> patch buffer k % kFwdBufs (tid 0)
-    auto load = [&](int t, int k) {
-        const int img = t / G.per_img, r = t - img * G.per_img;
-        const int tyi = r / G.ntx, txi = r - tyi * G.ntx;
-        const int b = k % kFwdBufs;
-        mbar_expect_tx(&full[b], 4 * kPlaneData);
-        issue_patch(&tmX, img, txi * TXP, tyi * TYP, sP0 + b * kPatch, &full[b]);
-    };
-    int issued = -1, consumed = -1;  // iterations whose load tid 0 issued / waited for
-    if (tid == 0 && (int)blockIdx.x < G.total) {
-        load(blockIdx.x, 0);
-        issued = 0;
-    }
-    bool failed = false;
-    int prev = -1, i = 0;
-    for (int t = blockIdx.x;; t += gridDim.x, i++) {
-        const bool have = t < G.total;
-        // tile i+1 into buffer (i+1) % 3: it held tile i-2, whose MMAs and
-        // epilogue finished before the last barrier
-        if (have && tid == 0 && t + (int)gridDim.x < G.total) {
-            load(t + gridDim.x, i + 1);
-            issued = i + 1;
-        }
-        if (prev >= 0) {  // epilogue of the previous tile overlaps this tile's loads
-            const int j = i - 1;
-            const bool ok = mbar_wait_first(&mbar[j & 1], (j >> 1) & 1);
-            if (__syncthreads_or(!ok)) {
-                failed = true;
-                break;
-            }
-            fence_after();
-            // the staging area is the patch buffer of tile j, whose MMAs are done;
-            // the next TMA load into it comes after the barrier below (the proxy
-            // fence orders these generic accesses before that async write)
-            conv_epilogue(a, G, prev, tmem + (uint32_t)((j & 1) * 32), warp, lane, sBias,
-                          sP0 + (j % kFwdBufs) * kPatch);
-            fence_async_smem();
-        }
-        if (!have) break;
-        fence_before();
-        __syncthreads();
-        fence_after();
-        if (tid == 0 && mbar_wait_first(&full[i % kFwdBufs], (i / kFwdBufs) & 1)) {
-            consumed = i;
-            const uint32_t p_u32 = smem_u32(sP0 + (i % kFwdBufs) * kPatch);
-            const uint32_t d = tmem + (uint32_t)((i & 1) * 32);
-#pragma unroll 1
-            for (int tap = 0; tap < 9; tap++) {
-                const int dy = tap / 3, dx = tap - dy * 3;
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const uint64_t da = sdesc(p_u32 + 2 * h * kPlane + (dy * PW + dx) * 16, kPlane, PW * 16);
-                    const uint64_t db = sdesc(w_u32 + (tap * 4 + 2 * h) * 512, 512, 128);
-                    mma_bf16(d, da, db, id, (tap | h) ? 1u : 0u);
-                }
-            }
-            mma_commit(&mbar[i & 1]);
-        }
-        prev = t;
-    }
-    if (failed) {
-        if (tid == 0) {
-            atomicExch(&g_corr_err, 1);
-            // patch loads that may still run: issued but not waited for
-            for (int k = consumed + 1; k <= issued; k++) mbar_wait(&full[k % kFwdBufs], (k / kFwdBufs) & 1);
-        }
-        // the MMAs of the last issued tile may still run
-        mbar_wait(&mbar[(i - 1) & 1], ((i - 1) >> 1) & 1);
-    }
-    fence_before();
-    __syncthreads();
-    fence_after();
-    if (warp == 0) tmem_dealloc(tmem, 64);
-}
-
-// Warp-specialised forward convolution (same tiles, operands and epilogue as
-// conv3x3_fwd_kernel).  The CTA's tiles are t = blockIdx.x + k * gridDim.x.
-//   warp 0 (lane 0): tile k -> patch buffer k % kWsBufs once the MMAs of tile
-//     k - kWsBufs have released it (empty barrier), TMA, full barrier;
-//   warp 1 (lane 0): waits for the patch and for a free accumulator
-//     (tile k - kWsAcc's epilogue has read it), issues the 18 MMAs of tile k
-//     into accumulator k % kWsAcc and commits to the patch's empty barrier and
-//     the accumulator's full barrier;
-//   warps 2-5: wait for the accumulator, read their 32 TMEM lanes (warp w
-//     reads lanes 32 (w % 4) ..), release the accumulator, finish the tile.
-// No role waits at a CTA barrier inside the loop, so MMAs of tile k run
-// while tile k - 1's epilogue stores and tile k + 1..k + 5 load.  Every wait
-// is bounded; a role whose wait expires sets the error word and leaves its
-// loop, the others' waits then expire in turn, and before TMEM is freed the
-// producer waits for its issued-but-unconsumed patch loads and the MMA warp
-// for its last MMAs.
-__global__ void __launch_bounds__(kWsThreads) conv3x3_fwd_ws_kernel(ConvArgs a, const __grid_constant__ CUtensorMap tmX) {
-    extern __shared__ unsigned char sm_raw[];
-    unsigned char *sm = smem_align<1024>(sm_raw);
-    unsigned char *sW = sm;
-    unsigned char *sP0 = sm + kWBytes;                         // kWsBufs patch buffers
-    unsigned char *sStage = sP0 + kWsBufs * kPatch;            // 4 x 2 KB epilogue staging
-    uint64_t *full = reinterpret_cast<uint64_t *>(sStage + kWsStage);  // [kWsBufs] patch landed
-    uint64_t *empty = full + kWsBufs;                                  // [kWsBufs] patch's MMAs done
-    uint64_t *accf = empty + kWsBufs;                                  // [kWsAcc] accumulator ready
-    uint64_t *acce = accf + kWsAcc;                                    // [kWsAcc] accumulator read
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(acce + kWsAcc);
-    int *sCount = reinterpret_cast<int *>(tslot + 1);  // [0] loads issued, [1] patches consumed
-    __shared__ float sBias[32];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const TileGeom G = tile_geom(a.nimg, a.H, a.W);
-    const int ntile = (int)blockIdx.x < G.total ? (G.total - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-
-    for (int c = tid; c < 32 * 36; c += kWsThreads) {
-        const int n = c / 36, r = c - n * 36;  // r = tap * 4 + quarter
-        cp_async16(sW + r * 512 + n * 16, a.Wk + n * KROWS + r * 8, 16);
-    }
-    cp_async_commit();
-    if (tid < 32) sBias[tid] = a.bias ? a.bias[tid] : 0.f;
-    if (warp == 1) tmem_alloc(tslot, 32 * kWsAcc);
-    if (tid == 0) {
-        for (int k = 0; k < kWsBufs; k++) {
+        for (int k = 0; k < kChunks; k++) {
             mbar_init(&full[k], 1);
             mbar_init(&empty[k], 1);
         }
-        for (int k = 0; k < kWsAcc; k++) {
+        for (int k = 0; k < kAcc; k++) {
             mbar_init(&accf[k], 1);
-            mbar_init(&acce[k], 4);  // one arrival per epilogue warp
+            mbar_init(&acce[k], 4);  // one arrival per lane quarter
         }
+        mbar_init(fin, 1);
         sCount[0] = sCount[1] = 0;
         mbar_init_fence();
     }
@@ -484,251 +390,379 @@ __global__ void __launch_bounds__(kWsThreads) conv3x3_fwd_ws_kernel(ConvArgs a, 
     __syncthreads();
     fence_after();
     const uint32_t tmem = *tslot;
+    Segments seg(a.H, G.rows, blockIdx.x, gridDim.x);
 
     if (warp == 0) {
-        if (lane == 0) {
-            int k = 0;
-            for (; k < ntile; k++) {
-                const int b = k % kWsBufs;
-                if (k >= kWsBufs && !mbar_wait_first(&empty[b], ((k / kWsBufs) - 1) & 1)) {
-                    atomicExch(&g_corr_err, 1);
-                    break;
-                }
-                const int t = (int)blockIdx.x + k * (int)gridDim.x;
-                const int img = t / G.per_img, r = t - img * G.per_img;
-                const int tyi = r / G.ntx, txi = r - tyi * G.ntx;
-                mbar_expect_tx(&full[b], 4 * kPlaneData);
-                issue_patch(&tmX, img, txi * TXP, tyi * TYP, sP0 + b * kPatch, &full[b]);
+        int c = 0;  // chunks issued
+        bool ok = true;
+        while (ok && seg.next()) {
+            const int g = seg.set * NG + lane, ng = min(NG, G.groups - seg.set * NG);
+            const int img = g / G.ntx, x0 = (g - img * G.ntx) * GX;
+            for (int r = seg.y0 - 1; r <= seg.y1 && ok; r += kCRows, c++) {
+                const int b = c % kChunks;
+                if (c >= kChunks) ok = mbar_wait_first(&empty[b], ((c / kChunks) - 1) & 1);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                if (lane == 0) mbar_expect_tx(&full[b], ng * kGrpBytes);
+                __syncwarp();
+                if (lane < ng) tma_load_4d(sP + b * kChunk + lane * kGrpBytes, &tmX, 0, x0 - 1, r, img, &full[b]);
             }
-            sCount[0] = k;
+        }
+        if (lane == 0) {
+            if (!ok) atomicExch(&g_corr_err, 1);
+            sCount[0] = c;
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t id = idesc(128, 32, 0, 0);
-            const uint32_t w_u32 = smem_u32(sW);
-            int k = 0;
-            for (; k < ntile; k++) {
-                const int b = k % kWsBufs, ac = k % kWsAcc;
-                if (!mbar_wait_first(&full[b], (k / kWsBufs) & 1)) {
-                    atomicExch(&g_corr_err, 1);
-                    break;
+        const uint64_t db0 = sdesc(smem_u32(sW), kWBlk, 128);
+        const uint64_t dp0 = sdesc64(smem_u32(sP), 16, kGrpBytes);  // an address is the descriptor's low bits
+        int cb = -1, chunks = 0;  // current chunk's ring slot, chunks waited for
+        unsigned cph = 1;         // parity of the current pass over the chunk ring
+        int sh = 0;               // accumulator slot of the next fresh output row
+        unsigned aph = 1;         // parity of a read accumulator on this pass (1 at first: a fresh barrier)
+        bool ok = true;
+        while (ok && seg.next()) {
+            int in = kCRows;  // row of the current chunk
+            for (int r = seg.y0 - 1; r <= seg.y1; r++, in++) {
+                if (in == kCRows) {
+                    in = 0;
+                    cb = (cb == kChunks - 1) ? 0 : cb + 1;
+                    if (cb == 0) cph ^= 1;
+                    ok = mbar_wait_first(&full[cb], cph);
+                    if (__any_sync(0xffffffffu, !ok)) {
+                        ok = false;
+                        break;
+                    }
+                    chunks++;
                 }
-                sCount[1] = k + 1;
-                if (k >= kWsAcc && !mbar_wait_first(&acce[ac], ((k / kWsAcc) - 1) & 1)) {
-                    atomicExch(&g_corr_err, 1);
-                    break;
+                // output rows lo .. hi take part; hi is fresh (no contribution yet) if it is r + 1
+                const int lo = max(r - 1, seg.y0), hi = min(r + 1, seg.y1 - 1), nl = hi - lo + 1;
+                const bool fresh = hi == r + 1;
+                const int sl = (sh - (fresh ? nl - 1 : nl)) & (kAcc - 1);  // slot of lo
+                if (fresh) {
+                    ok = mbar_wait_first(&acce[sh], aph);
+                    if (__any_sync(0xffffffffu, !ok)) {
+                        ok = false;
+                        break;
+                    }
+                    sh = (sh + 1) & (kAcc - 1);
+                    if (sh == 0) aph ^= 1;
                 }
                 fence_after();
-                const uint32_t p_u32 = smem_u32(sP0 + b * kPatch);
-                const uint32_t d = tmem + (uint32_t)(ac * 32);
-#pragma unroll 1
-                for (int tap = 0; tap < 9; tap++) {
-                    const int dy = tap / 3, dx = tap - dy * 3;
+                const uint64_t da0 = dp0 + (uint64_t)(uint32_t)((cb * kChunk + in * kGRow) >> 4);
+                // outputs lo + [i, j) of this input row, whose accumulators
+                // start at slot s; dx, h: column offset and channel half; blk:
+                // lo's block of the weights
+                auto mma = [&](int blk, int dx, int h, int i, int j, int s, uint32_t acc) {
+                    mma_bf16(tmem + (uint32_t)(s * 32), da0 + (uint64_t)((dx * kPix + h * 32) >> 4),
+                             db0 + (uint64_t)(((dx * 4 + 2 * h) * kWBlk + (blk + i) * 512) >> 4),
+                             idesc(128, 32 * (j - i), 0, 0), acc);
+                };
+                if (elect_one()) {
+                    // the usual cases straight: the issuing lane's instructions
+                    // are what the tensor pipe waits for
+                    if (fresh && nl == 3 && sl <= kAcc - 3) {
+                        mma(0, 0, 0, 0, 2, sl, 1u);
+                        mma(0, 0, 0, 2, 3, sl + 2, 0u);
 #pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        const uint64_t da = sdesc(p_u32 + 2 * h * kPlane + (dy * PW + dx) * 16, kPlane, PW * 16);
-                        const uint64_t db = sdesc(w_u32 + (tap * 4 + 2 * h) * 512, 512, 128);
-                        mma_bf16(d, da, db, id, (tap | h) ? 1u : 0u);
+                        for (int t = 1; t < 6; t++) mma(0, t >> 1, t & 1, 0, 3, sl, 1u);
+                    } else if (fresh && nl == 3 && sl == kAcc - 2) {
+#pragma unroll
+                        for (int t = 0; t < 6; t++) {
+                            mma(0, t >> 1, t & 1, 0, 2, sl, 1u);
+                            mma(0, t >> 1, t & 1, 2, 3, 0, t ? 1u : 0u);
+                        }
+                    } else if (fresh && nl == 3) {
+                        mma(0, 0, 0, 0, 1, sl, 1u);
+                        mma(0, 0, 0, 1, 2, 0, 1u);
+                        mma(0, 0, 0, 2, 3, 1, 0u);
+#pragma unroll
+                        for (int t = 1; t < 6; t++) {
+                            mma(0, t >> 1, t & 1, 0, 1, sl, 1u);
+                            mma(0, t >> 1, t & 1, 1, 3, 0, 1u);
+                        }
+                    } else {  // a segment's first and last rows: row by row
+                        const int blk = lo - (r - 1);
+#pragma unroll 1
+                        for (int t = 0; t < 6; t++)
+#pragma unroll 1
+                            for (int i = 0; i < nl; i++)
+                                mma(blk, t >> 1, t & 1, i, i + 1, (sl + i) & (kAcc - 1),
+                                    (fresh && t == 0 && i == nl - 1) ? 0u : 1u);
                     }
+                    if (in == kCRows - 1 || r == seg.y1) mma_commit(&empty[cb]);
+                    if (r - 1 >= seg.y0) mma_commit(&accf[sl]);  // output row r - 1 is complete
                 }
-                mma_commit(&empty[b]);
-                mma_commit(&accf[ac]);
+                __syncwarp();
             }
-            // the MMAs issued last may still run: they signal the last
-            // accumulator's full barrier when done
-            if (k > 0) mbar_wait(&accf[(k - 1) % kWsAcc], ((k - 1) / kWsAcc) & 1);
+        }
+        if (elect_one()) {
+            if (!ok) atomicExch(&g_corr_err, 1);
+            sCount[1] = chunks;
+            mma_commit(fin);
+            mbar_wait(fin, 0);
         }
     } else {
-        const int q = warp & 3;  // TMEM lane quarter this warp may read
-        for (int k = 0; k < ntile; k++) {
-            const int ac = k % kWsAcc;
-            // every lane waits; the warp leaves together if any lane's wait
-            // expired (the TMEM load below is a warp-wide instruction)
-            const bool ok = mbar_wait_first(&accf[ac], (k / kWsAcc) & 1);
-            if (__any_sync(0xffffffffu, !ok)) {
-                if (lane == 0) atomicExch(&g_corr_err, 1);
-                break;
+        const int q = warp & 3;                  // TMEM lane quarter this warp may read
+        const int par = (warp - 2) >> 2;         // output rows this warp takes: k % (kEpiWarps / 4)
+        uint4 *sw = reinterpret_cast<uint4 *>(sStage + (warp - 2) * 2048);
+        int k = 0;
+        bool ok = true;
+        while (ok && seg.next()) {
+            // groups 4 q .. 4 q + 3 of the set: this lane's own pixel, and the
+            // pixel and chunk it stores of each
+            long long px = -1, row[4];
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const int g = seg.set * NG + 4 * q + r;
+                const int img = g / G.ntx, x0 = (g - img * G.ntx) * GX;
+                const long long o = (long long)img * a.H * a.W;
+                const int xr = x0 + (lane >> 2), xo = x0 + (lane & 7);
+                row[r] = (g < G.groups && xr < a.W) ? (o + xr) * C + (lane & 3) * 8 : -1;
+                if ((lane >> 3) == r && g < G.groups && xo < a.W) px = (o + xo) * C;
             }
-            fence_after();
-            const int t = (int)blockIdx.x + k * (int)gridDim.x;
-            conv_epilogue(a, G, t, tmem + (uint32_t)(ac * 32), q, lane, sBias, sStage, &acce[ac]);
+            for (int y = seg.y0; y < seg.y1; y++, k++) {
+                if (k % (kEpiWarps / 4) != par) continue;
+                const int ac = k % kAcc;
+                // every lane waits; the warp leaves together if any lane's wait
+                // expired (the TMEM load below is a warp-wide instruction)
+                ok = mbar_wait_first(&accf[ac], (k / kAcc) & 1);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                fence_after();
+                conv_epilogue(a, y, tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(ac * 32), lane, sBias, sw, px, row,
+                              &acce[ac]);
+            }
         }
+        if (!ok && lane == 0) atomicExch(&g_corr_err, 1);
     }
     __syncwarp();
     fence_before();
     __syncthreads();
-    if (tid == 0) {  // patch loads issued but never consumed (an expired wait): let them land
-        for (int k = sCount[1]; k < sCount[0]; k++) mbar_wait(&full[k % kWsBufs], (k / kWsBufs) & 1);
+    if (tid == 0) {  // chunks issued but never waited for (an expired wait): let them land
+        for (int c = sCount[1]; c < sCount[0]; c++) mbar_wait(&full[c % kChunks], (c / kChunks) & 1);
     }
     __syncthreads();
     fence_after();
-    if (warp == 1) tmem_dealloc(tmem, 32 * kWsAcc);
+    if (warp == 1) tmem_dealloc(tmem, 32 * kAcc);
 }
 
-// Weight (and bias) gradient partials of this CTA's strip of tiles, written
-// to its row of `part` ([gridDim.x][kWgPart]: dW[cout][288], then the 4 warps'
-// bias sums [4][32]); wgrad_reduce_kernel adds the rows to dW and db in a
-// fixed order, so the gradient does not depend on which CTA finishes first.
+struct TileGeom {
+    int ntx, nty, per_img, total;
+};
+__host__ __device__ inline TileGeom tile_geom(int nimg, int H, int W) {
+    TileGeom g;
+    g.ntx = (W + GX - 1) / GX;
+    g.nty = (H + TYP - 1) / TYP;
+    g.per_img = g.ntx * g.nty;
+    g.total = nimg * g.per_img;
+    return g;
+}
+
+// Weight (and bias) gradient partials of this CTA's tiles, written to its row
+// of `part` ([gridDim.x][kWgPart]: dW[cout][288], then the 4 warps' bias sums
+// [4][32]); wgrad_reduce_kernel adds the rows to dW and db in a fixed order, so
+// the gradient does not depend on which CTA finishes first.
+//   warp 0: tile k (8 x 16 pixels) of X with one row of halo above and below,
+//     and of dZ with one column left and right, into a ring of kWgStages;
+//   warp 1 (lane 0): per 16 pixels (two tile rows) one MMA of
+//     D[dy * 32 + cin (+ 32 ignored rows)][j * 32 + cout], j = 1 - dx:
+//     A = X shifted by dy rows (blocks one tile row apart), B = dZ shifted by j
+//     columns (blocks one pixel apart: overlapping windows of the same tile).
+//     X[p'] dZ[p' - dx] summed over p' is the tap's gradient: both operands
+//     are zero outside the image;
+//   warps 2-5: the bias gradient on the CUDA cores, a pixel per thread.
 constexpr int kWgPart = 32 * KROWS + 4 * 32;
-__global__ void __launch_bounds__(128, kWgCtasPerSm)
-    conv3x3_wgrad_kernel(const __grid_constant__ CUtensorMap tmXr, const __grid_constant__ CUtensorMap tmZ, int nimg,
+__global__ void __launch_bounds__(kWgThreads, 1)
+    conv3x3_wgrad_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmZ, int nimg,
                          int H, int W, float *__restrict__ part) {
     extern __shared__ unsigned char sm_raw[];
-    unsigned char *sm = smem_align<1024>(sm_raw);  // two stages: patch (12288 B) + dZ planes (4 x 2048 B)
-    uint64_t *full = reinterpret_cast<uint64_t *>(sm + 2 * kWgStage);  // [2] stage loaded
-    uint64_t *done = full + 2;                                          // [2] MMAs of the stage finished
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(full + 4);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    unsigned char *sm = smem_align<1024>(sm_raw);
+    uint64_t *full = reinterpret_cast<uint64_t *>(sm + kWgStages * kWgStage);  // [kWgStages] stage loaded
+    uint64_t *empty = full + kWgStages;  // [kWgStages] stage's MMAs and bias sums done
+    uint64_t *accf = empty + kWgStages;  // [2] accumulator set's batch summed
+    uint64_t *acce = accf + 2;           // [2] accumulator set read
+    uint64_t *fin = acce + 2;            // all MMAs done
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(fin + 1);
+    int *sCount = reinterpret_cast<int *>(tslot + 1);  // [0] stages issued, [1] stages waited for by the MMA warp
+    int *sFail = sCount + 2;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const TileGeom G = tile_geom(nimg, H, W);
+    const int ntile = (int)blockIdx.x < G.total ? (G.total - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
 
-    if (warp == 0) tmem_alloc(tslot, 128);
+    if (warp == 1) tmem_alloc(tslot, 256);
     if (tid == 0) {
-        for (int k = 0; k < 4; k++) mbar_init(&full[k], 1);
+        for (int k = 0; k < 2; k++) {
+            mbar_init(&accf[k], 1);
+            mbar_init(&acce[k], 4);
+        }
+        for (int k = 0; k < kWgStages; k++) {
+            mbar_init(&full[k], 1);
+            mbar_init(&empty[k], 5);  // the MMAs and four bias warps
+        }
+        mbar_init(fin, 1);
+        sCount[0] = sCount[1] = 0;
+        *sFail = 0;
         mbar_init_fence();
     }
     fence_before();
     __syncthreads();
     fence_after();
     const uint32_t tmem = *tslot;
-    const uint32_t id = idesc(128, 32, 1, 1);
-    const uint32_t sm_u32 = smem_u32(sm);
-
-    // tile t -> stage st: the patch (one 5-D box, zero fill outside the
-    // image) and the dZ tile (four channel-quarter boxes)
-    auto issue = [&](int t, int st) {
-        const int img = t / G.per_img, r = t - img * G.per_img;
-        const int tyi = r / G.ntx, txi = r - tyi * G.ntx;
-        const int x0 = txi * TXP, y0 = tyi * TYP;
-        unsigned char *stg = sm + st * kWgStage;
-        mbar_expect_tx(&full[st], kWgPatch + 4 * kZPlane);
-        tma_load_5d(stg, &tmXr, 0, x0 - 1, 0, y0 - 1, img, &full[st]);
+    float db[32];      // bias gradient of this thread's pixels
+    float sum[3][32];  // this lane's row of D (j, cout), summed over the batches
 #pragma unroll
-        for (int q = 0; q < 4; q++) tma_load_4d(stg + kWgPatchBuf + q * kZPlane, &tmZ, 8 * q, x0, y0, img, &full[st]);
-    };
-    // for the error path (tid 0): the last iteration whose load was issued, the
-    // last whose load was waited for, and the last whose MMAs were committed
-    int last_load = -1, consumed = -1, last_mma = -1;
-    if (tid == 0 && (int)blockIdx.x < G.total) {
-        issue(blockIdx.x, 0);
-        last_load = 0;
-    }
-    float dbp[8];  // bias gradient partials: cout q * 8 + 2 * (lane & 3) + {0, 1}
-#pragma unroll
-    for (int k = 0; k < 8; k++) dbp[k] = 0.f;
+    for (int n = 0; n < 32; n++) db[n] = sum[0][n] = sum[1][n] = sum[2][n] = 0.f;
 
-    bool failed = false;
-    int i = 0;
-    for (int t = blockIdx.x; t < G.total; t += gridDim.x, i++) {
-        const int b = i & 1;
-        // first the next tile into the other stage, once the MMAs of the tile
-        // it held have finished (its bias reads ended at the last barrier),
-        // so that two loads are in flight while this tile waits for its data
+    if (warp == 0) {
+        if (lane == 0) {
+            int k = 0;
+            for (; k < ntile; k++) {
+                const int b = k % kWgStages;
+                if (k >= kWgStages && !mbar_wait_first(&empty[b], ((k / kWgStages) - 1) & 1)) {
+                    atomicExch(sFail, 1);
+                    break;
+                }
+                const int t = (int)blockIdx.x + k * (int)gridDim.x;
+                const int img = t / G.per_img, r = t - img * G.per_img;
+                const int tyi = r / G.ntx, x0 = (r - tyi * G.ntx) * GX, y0 = tyi * TYP;
+                unsigned char *stg = sm + b * kWgStage;
+                mbar_expect_tx(&full[b], kXBytes + kZBytes);
+                tma_load_4d(stg, &tmX, 0, x0, y0 - 1, img, &full[b]);
+                tma_load_4d(stg + kXBuf, &tmZ, 0, x0 - 1, y0, img, &full[b]);
+            }
+            sCount[0] = k;
+        }
+    } else if (warp == 1) {
+        const uint32_t id = idesc(128, 96, 1, 1);
+        const uint64_t dx0 = sdesc64(smem_u32(sm), kXRow, kXRow);  // an address is the descriptor's low bits
+        const uint64_t dz0 = sdesc64(smem_u32(sm) + kXBuf, kPix, kGRow);
+        int b = 0, first = 0, f = 0, k = 0;  // ring slot; tile of the batch, batch; tile
+        unsigned ph = 0;
         bool ok = true;
-        const int tn = t + gridDim.x;
-        if (tid == 0 && tn < G.total) {
-            if (i >= 1) ok = mbar_wait_first(&done[b ^ 1], ((i - 1) >> 1) & 1);
-            if (ok) {
-                issue(tn, b ^ 1);
-                last_load = i + 1;
-            }
-        }
-        const bool loaded = mbar_wait_first(&full[b], (i >> 1) & 1);
-        if (__syncthreads_or(!loaded || !ok)) {
-            failed = true;
-            break;
-        }
-        consumed = i;
-        if (tid == 0) {
-            // D[dy * 32 + cin (+ 32 ignored rows)][cout] for each dx: A = the
-            // shifted patch (M groups (dy, quarter) 160 B apart, K groups =
-            // tile rows 640 B apart), B = dZ (N groups = quarters, K groups =
-            // tile rows 128 B apart); 16 pixels (two tile rows) per MMA
-            const uint32_t pb = sm_u32 + b * kWgStage, zb = pb + kWgPatchBuf;
-#pragma unroll 1
-            for (int s = 0; s < 8; s++) {
-                const uint64_t dz = sdesc(zb + s * 256, 128, kZPlane);
-#pragma unroll
-                for (int dx = 0; dx < 3; dx++) {
-                    const uint64_t da = sdesc(pb + s * 2 * kRowQ + dx * 16, kRowQ, PW * 16);
-                    mma_bf16(tmem + (uint32_t)(dx * 32), da, dz, id, (i > 0 || s > 0) ? 1u : 0u);
-                }
-            }
-            mma_commit(&done[b]);
-            last_mma = i;
-        }
-        // bias gradient from the dZ tile: per instruction a warp reads 32
-        // consecutive words (8 pixels x 16 B), no bank conflicts
-        const unsigned char *zt = sm + b * kWgStage + kWgPatchBuf;
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-#pragma unroll
-            for (int pb8 = 0; pb8 < 4; pb8++) {
-                const int px = warp * 32 + pb8 * 8 + (lane >> 2);
-                const __nv_bfloat162 v =
-                    *reinterpret_cast<const __nv_bfloat162 *>(zt + q * kZPlane + px * 16 + (lane & 3) * 4);
-                dbp[2 * q] += __low2float(v);
-                dbp[2 * q + 1] += __high2float(v);
-            }
-        }
-        fence_async_smem();  // this stage's generic reads before a later TMA write into it
-        __syncthreads();
-    }
-    const int n = i;  // iterations entered (the last may have failed)
-    float *prow = part + (size_t)blockIdx.x * kWgPart;
-    if (failed || n == 0)  // no partials from this CTA
-        for (int k = tid; k < kWgPart; k += 128) prow[k] = 0.f;
-    if (failed) {
-        if (tid == 0) {
-            atomicExch(&g_corr_err, 1);
-            // whatever may still run: the last load and the last MMAs
-            // loads issued but not waited for (up to two: this tile's and the next)
-            for (int k = consumed + 1; k <= last_load; k++) mbar_wait(&full[k & 1], (k >> 1) & 1);
-            // the last commit covers every earlier MMA of this thread
-            if (last_mma >= 0) mbar_wait(&done[last_mma & 1], (last_mma >> 1) & 1);
-        }
-    } else if (n > 0) {
-        const int L = n - 1;
-        const bool ok = mbar_wait_first(&done[L & 1], (L >> 1) & 1);
-        if (__syncthreads_or(!ok)) {
-            for (int k = tid; k < kWgPart; k += 128) prow[k] = 0.f;
-            if (tid == 0) {
-                atomicExch(&g_corr_err, 1);
-                mbar_wait(&done[L & 1], (L >> 1) & 1);  // the MMAs before TMEM is freed
-            }
-        } else {
+        for (; k < ntile; k++) {
+            ok = mbar_wait_first(&full[b], ph);
+            if (first == 0 && f >= 2) ok &= mbar_wait_first(&acce[f & 1], ((f >> 1) - 1) & 1);
+            if (__any_sync(0xffffffffu, !ok)) break;
             fence_after();
-            if (warp < 3) {  // rows 0..95: dy = warp, cin = lane; rows 96..127 are ignored
-#pragma unroll 1
-                for (int dx = 0; dx < 3; dx++) {
-                    float v[32];
-                    tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(dx * 32), v);
-                    const int m = (warp * 3 + dx) * 32 + lane;  // tap * 32 + cin
+            const uint64_t st = (uint64_t)(uint32_t)((b * kWgStage) >> 4), da = dx0 + st, dz = dz0 + st;
+            const uint32_t d = tmem + (uint32_t)((f & 1) * 128);
+            if (elect_one()) {
+                mma_bf16(d, da, dz, id, first ? 1u : 0u);
 #pragma unroll
-                    for (int c = 0; c < 32; c++) prow[c * KROWS + m] = v[c];
-                }
+                for (int s = 1; s < TYP / 2; s++)
+                    mma_bf16(d, da + (uint64_t)((2 * s * kXRow) >> 4), dz + (uint64_t)((2 * s * kGRow) >> 4), id, 1u);
+                mma_commit(&empty[b]);
+                if (first == kWgFlush - 1 || k == ntile - 1) mma_commit(&accf[f & 1]);
             }
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                float v = dbp[k];
-                v += __shfl_xor_sync(0xffffffffu, v, 4);
-                v += __shfl_xor_sync(0xffffffffu, v, 8);
-                v += __shfl_xor_sync(0xffffffffu, v, 16);
-                dbp[k] = v;
+            __syncwarp();
+            if (++b == kWgStages) {
+                b = 0;
+                ph ^= 1;
             }
-            if (lane < 4) {
-                float *pb = prow + 32 * KROWS + warp * 32;
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    pb[q * 8 + 2 * lane] = dbp[2 * q];
-                    pb[q * 8 + 2 * lane + 1] = dbp[2 * q + 1];
-                }
+            if (++first == kWgFlush) {
+                first = 0;
+                f++;
             }
         }
+        if (elect_one()) {
+            if (k < ntile) atomicExch(sFail, 1);
+            sCount[1] = k;
+            mma_commit(fin);
+            mbar_wait(fin, 0);
+        }
+    } else {
+        const int p = tid - 64;  // pixel of the tile: 8 per row
+        const uint32_t off = (p >> 3) * kGRow + ((p & 7) + 1) * kPix;
+        const int dy = warp & 3;  // TMEM lanes 32 dy ..: rows dy * 32 + cin; dy = 3 is ignored
+        // adds batch f's accumulators to `sum` and hands them back
+        auto flush = [&](int f) {
+            const bool ok = mbar_wait_first(&accf[f & 1], (f >> 1) & 1);
+            if (__any_sync(0xffffffffu, !ok)) return false;
+            fence_after();
+            if (dy < 3) {
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    float v[32];
+                    tmem_ld32(tmem + ((uint32_t)(dy * 32) << 16) + (uint32_t)((f & 1) * 128 + j * 32), v);
+#pragma unroll
+                    for (int n = 0; n < 32; n++) sum[j][n] += v[n];
+                }
+            }
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acce[f & 1]);
+            return true;
+        };
+        int flushed = 0;  // batches
+        bool good = true;
+        for (int k = 0; k < ntile; k++) {
+            const int b = k % kWgStages;
+            // the batch before this one's, once the MMAs are well into this one
+            if (k >= flushed * kWgFlush + kWgFlush + kWgFlush / 2) good = flush(flushed++);
+            const bool ok = good && mbar_wait_first(&full[b], (k / kWgStages) & 1);
+            if (__any_sync(0xffffffffu, !ok)) {
+                if (lane == 0) atomicExch(sFail, 1);
+                good = false;
+                break;
+            }
+            const unsigned char *z = sm + b * kWgStage + kXBuf + off;
+            const uint32_t swz = (smem_u32(z) >> 7) & 3;
+            uint4 v[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) v[c] = *reinterpret_cast<const uint4 *>(z + ((c ^ swz) << 4));
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const uint32_t w[4] = {v[c].x, v[c].y, v[c].z, v[c].w};
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162 *>(&w[j]);
+                    db[8 * c + 2 * j] += __low2float(h);
+                    db[8 * c + 2 * j + 1] += __high2float(h);
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[b]);
+        }
+        while (good && flushed * kWgFlush < ntile) good = flush(flushed++);
+        if (!good && lane == 0) atomicExch(sFail, 1);
+    }
+    __syncwarp();
+    fence_before();
+    __syncthreads();
+    if (tid == 0) {
+        if (*sFail) atomicExch(&g_corr_err, 1);
+        // stages issued but never waited for (an expired wait): let them land
+        for (int k = sCount[1]; k < sCount[0]; k++) mbar_wait(&full[k % kWgStages], (k / kWgStages) & 1);
+    }
+    __syncthreads();
+    fence_after();
+    float *prow = part + (size_t)blockIdx.x * kWgPart;
+    if (*sFail || ntile == 0) {  // no partials from this CTA
+        for (int k = tid; k < kWgPart; k += kWgThreads) prow[k] = 0.f;
+    } else if (warp >= 2) {
+        const int dy = warp & 3;
+        if (dy < 3) {
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                const int m = (dy * 3 + 2 - j) * 32 + lane;  // tap * 32 + cin
+#pragma unroll
+                for (int n = 0; n < 32; n++) prow[n * KROWS + m] = sum[j][n];
+            }
+        }
+        float mine = 0.f;  // channel `lane` summed over the warp's 32 pixels
+#pragma unroll
+        for (int n = 0; n < 32; n++) {
+            float v = db[n];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == n) mine = v;
+        }
+        prow[32 * KROWS + (warp - 2) * 32 + lane] = mine;
     }
     fence_before();
     __syncthreads();
     fence_after();
-    if (warp == 0) tmem_dealloc(tmem, 128);
+    if (warp == 1) tmem_dealloc(tmem, 256);
 }
 
 // ---------------------------------------------------------------- training
@@ -929,16 +963,16 @@ __global__ void apply_kernel(const float *__restrict__ Y, const float *__restric
 }
 
 // tensor map of an NHWC BF16 32-channel tensor [nimg][H][W][32] with boxes of
-// 8 channels x bx x by pixels
+// 32 channels x bx x by pixels, 64-byte swizzle (dst multiples of 512 B)
 cudaError_t make_map(CUtensorMap *m, const void *base, int nimg, int H, int W, int bx, int by) {
     EncodeTiledFn f = tensor_map_encoder();
     if (!f) return cudaErrorNotSupported;
     const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)nimg};
     const cuuint64_t strides[3] = {(cuuint64_t)C * 2, (cuuint64_t)C * 2 * W, (cuuint64_t)C * 2 * W * H};
-    const cuuint32_t box[4] = {8, (cuuint32_t)bx, (cuuint32_t)by, 1};
+    const cuuint32_t box[4] = {C, (cuuint32_t)bx, (cuuint32_t)by, 1};
     const cuuint32_t es[4] = {1, 1, 1, 1};
     const CUresult r = f(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(base), dims, strides, box, es,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
@@ -947,8 +981,6 @@ cudaError_t prepare() {
     static bool done = false;
     if (done) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(conv3x3_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(conv3x3_fwd_ws_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWsSmem);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(conv3x3_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem);
     if (e == cudaSuccess) done = true;
@@ -965,74 +997,97 @@ int num_sms() {
     return n;
 }
 
-// The warp-specialised forward kernel is the default (8 x 512^2 images, BF16
-// output with ReLU: 405 vs 383 TFLOP/s on one box); TSU_CONV_FWD=plain
-// selects conv3x3_fwd_kernel, whose four CTAs per SM each alternate MMAs and
-// epilogue.
-bool fwd_ws() {
-    static const bool ws = [] {
-        const char *e = std::getenv("TSU_CONV_FWD");
-        return !(e && !std::strcmp(e, "plain"));
-    }();
-    return ws;
-}
-
 cudaError_t conv_launch(const ConvArgs &a, cudaStream_t st) {
     cudaError_t e = prepare();
     if (e != cudaSuccess) return e;
     if (reinterpret_cast<uintptr_t>(a.X) % 16) return cudaErrorInvalidValue;
     CUtensorMap mx;
-    e = make_map(&mx, a.X, a.nimg, a.H, a.W, PW, PH);
+    e = make_map(&mx, a.X, a.nimg, a.H, a.W, GW, kCRows);
     if (e != cudaSuccess) return e;
-    const TileGeom G = tile_geom(a.nimg, a.H, a.W);
-    if (fwd_ws()) {  // persistent CTAs, kWsCtasPerSm per SM
-        const int ctas = std::min(G.total, kWsCtasPerSm * num_sms());
-        conv3x3_fwd_ws_kernel<<<ctas, kWsThreads, kWsSmem, st>>>(a, mx);
-        return cudaGetLastError();
-    }
-    // persistent CTAs, kFwdCtasPerSm per SM (shared memory and TMEM bound)
-    const int ctas = std::min(G.total, kFwdCtasPerSm * num_sms());
-    conv3x3_fwd_kernel<<<ctas, 128, kFwdSmem, st>>>(a, mx);
+    // persistent CTAs; at least two output rows each (every segment also reads
+    // the rows above and below it)
+    const int ctas = std::max(1, std::min(fwd_geom(a.nimg, a.H, a.W).rows / 2, kFwdCtas * num_sms()));
+    conv3x3_fwd_kernel<<<ctas, kFwdThreads, kFwdSmem, st>>>(a, mx);
     return cudaGetLastError();
 }
 
-// The NHWC tensor viewed as [n][y][channel quarter][x][8 channels] (dims
-// innermost first: 8 channels, x at 64 B, quarter at 16 B, y, n): a PW x PH
-// box lands in shared memory as [row][quarter][x][8], the weight gradient's
-// A operand layout.
-cudaError_t make_map_rowq(CUtensorMap *m, const void *base, int nimg, int H, int W) {
-    EncodeTiledFn f = tensor_map_encoder();
-    if (!f) return cudaErrorNotSupported;
-    const cuuint64_t dims[5] = {8, (cuuint64_t)W, 4, (cuuint64_t)H, (cuuint64_t)nimg};
-    const cuuint64_t strides[4] = {(cuuint64_t)C * 2, 16, (cuuint64_t)C * 2 * W, (cuuint64_t)C * 2 * W * H};
-    const cuuint32_t box[5] = {8, (cuuint32_t)PW, 4, (cuuint32_t)PH, 1};
-    const cuuint32_t es[5] = {1, 1, 1, 1, 1};
-    const CUresult r = f(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void *>(base), dims, strides, box, es,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
-}
-
-// dW[k] += sum over CTAs b (in order) of part[b][k]; db[n] += sum over b and
-// the 4 warps (in order) of the bias partials
-__global__ void wgrad_reduce_kernel(const float *__restrict__ part, int nctas, float *__restrict__ dW,
-                                    float *__restrict__ db) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < 32 * KROWS) {
-        float acc = 0.f;
-        for (int b = 0; b < nctas; b++) acc += part[(size_t)b * kWgPart + k];
-        dW[k] += acc;
-    } else if (db && k < 32 * KROWS + 32) {
-        const int n = k - 32 * KROWS;
-        float acc = 0.f;
-        for (int b = 0; b < nctas; b++)
-            for (int w = 0; w < 4; w++) acc += part[(size_t)b * kWgPart + 32 * KROWS + w * 32 + n];
-        db[n] += acc;
+// dW[k] += sum over CTAs of part[b][k]; db[n] += sum over CTAs and the 4 warps
+// of the bias partials.  A block owns 32 elements; each of its kRedWarps warps
+// takes every kRedWarps-th row (all loads in flight together: the kernel is a
+// latency, not a bandwidth), then the sums are added in order.
+constexpr int kRedWarps = 16, kRedRows = 10;  // one pass covers 160 rows
+__global__ void __launch_bounds__(32 * kRedWarps) wgrad_reduce_kernel(const float *__restrict__ part, int nctas,
+                                                                      float *__restrict__ dW, float *__restrict__ db) {
+    __shared__ float sSum[kRedWarps][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int k = blockIdx.x * 32 + lane;
+    const bool bias = k >= 32 * KROWS;  // the last block
+    const int n = bias ? 4 * nctas : nctas;
+    float acc = 0.f;
+    for (int b0 = w; b0 < n; b0 += kRedWarps * kRedRows) {
+        float v[kRedRows];
+#pragma unroll
+        for (int i = 0; i < kRedRows; i++) {
+            const int b = b0 + i * kRedWarps;
+            const float *p = bias ? part + (size_t)(b >> 2) * kWgPart + 32 * KROWS + (b & 3) * 32 + lane
+                                  : part + (size_t)b * kWgPart + k;
+            v[i] = (b < n) ? __ldcg(p) : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < kRedRows; i++) acc += v[i];
+    }
+    sSum[w][lane] = acc;
+    __syncthreads();
+    if (w == 0) {
+#pragma unroll
+        for (int q = 1; q < kRedWarps; q++) acc += sSum[q][lane];
+        if (!bias) dW[k] += acc;
+        else if (db) db[lane] += acc;
     }
 }
 
-// CTAs of a weight-gradient launch (4 persistent CTAs per SM: 128 TMEM columns each)
-int wgrad_ctas(int nimg, int H, int W) { return std::min(tile_geom(nimg, H, W).total, kWgCtasPerSm * num_sms()); }
+// CTAs of a weight-gradient launch
+int wgrad_ctas(int nimg, int H, int W) { return std::min(tile_geom(nimg, H, W).total, num_sms()); }
+
+// Stream-ordered scratch of the calls that bring none.  The device's default
+// pool gives its memory back at every synchronisation, and the next call then
+// maps it again (600 us against 80 us for the gradient itself); this pool
+// keeps up to kKeep bytes (one unit of its growth).  tsu_corr_destroy returns them.
+constexpr unsigned long long kKeep = 32ull << 20;
+constexpr int kMaxDevices = 64;
+std::mutex g_pool_mu;
+cudaMemPool_t g_pool[kMaxDevices] = {};
+
+cudaError_t scratch_alloc(float **p, size_t bytes, cudaStream_t st) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (st && cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+    cudaMemPool_t pool = nullptr;
+    if (cap == cudaStreamCaptureStatusNone && dev < kMaxDevices) {
+        std::lock_guard<std::mutex> g(g_pool_mu);
+        if (!g_pool[dev]) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            unsigned long long keep = kKeep;
+            if (cudaMemPoolCreate(&g_pool[dev], &props) != cudaSuccess) {
+                cudaGetLastError();
+                g_pool[dev] = nullptr;
+            } else {
+                cudaMemPoolSetAttribute(g_pool[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+            }
+        }
+        pool = g_pool[dev];
+    }
+    return pool ? cudaMallocFromPoolAsync((void **)p, bytes, pool, st) : cudaMallocAsync((void **)p, bytes, st);
+}
+void scratch_trim(int dev) {
+    std::lock_guard<std::mutex> g(g_pool_mu);
+    if (dev >= 0 && dev < kMaxDevices && g_pool[dev]) cudaMemPoolTrimTo(g_pool[dev], 0);
+}
 
 // part: wgrad_ctas(...) * kWgPart floats of device scratch, or null (then
 // allocated on the stream for this call)
@@ -1042,20 +1097,20 @@ cudaError_t wgrad_launch(const bf16 *X, const bf16 *dZ, int nimg, int H, int W, 
     if (e != cudaSuccess) return e;
     if (reinterpret_cast<uintptr_t>(X) % 16 || reinterpret_cast<uintptr_t>(dZ) % 16) return cudaErrorInvalidValue;
     CUtensorMap mx, mz;
-    e = make_map_rowq(&mx, X, nimg, H, W);
-    if (e == cudaSuccess) e = make_map(&mz, dZ, nimg, H, W, TXP, TYP);
+    e = make_map(&mx, X, nimg, H, W, GX, TYP + 2);
+    if (e == cudaSuccess) e = make_map(&mz, dZ, nimg, H, W, GW, TYP);
     if (e != cudaSuccess) return e;
     const int ctas = wgrad_ctas(nimg, H, W);
     float *own = nullptr;
     if (!part) {
-        e = cudaMallocAsync((void **)&own, (size_t)ctas * kWgPart * sizeof(float), st);
+        e = scratch_alloc(&own, (size_t)ctas * kWgPart * sizeof(float), st);
         if (e != cudaSuccess) return e;
         part = own;
     }
-    conv3x3_wgrad_kernel<<<ctas, 128, kWgSmem, st>>>(mx, mz, nimg, H, W, part);
+    conv3x3_wgrad_kernel<<<ctas, kWgThreads, kWgSmem, st>>>(mx, mz, nimg, H, W, part);
     e = cudaGetLastError();
     if (e == cudaSuccess) {
-        wgrad_reduce_kernel<<<(32 * KROWS + 32 + 255) / 256, 256, 0, st>>>(part, ctas, dW, db);
+        wgrad_reduce_kernel<<<KROWS + 1, 32 * kRedWarps, 0, st>>>(part, ctas, dW, db);
         e = cudaGetLastError();
     }
     if (own) {
@@ -1311,6 +1366,7 @@ extern "C" int tsu_corr_destroy(TsuCorrector *c) {
     cudaSetDevice(c->device);
     if (c->st) cudaStreamSynchronize(c->st);
     free_all(c);
+    scratch_trim(c->device);
     delete c;
     return TSU_OK;
 }
