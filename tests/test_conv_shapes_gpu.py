@@ -74,3 +74,29 @@ def test_weight_gradient_work_split(n, h, w, no_tf32):
     assert float((dW - ref).norm() / ref.norm()) < 1e-4
     assert torch.allclose(dW.double(), ref, rtol=1e-4, atol=1e-4 * float(ref.abs().max()))
     assert torch.allclose(db.double(), z.sum(0), rtol=1e-4, atol=1e-4 * float(z.sum(0).abs().max()))
+
+
+@pytest.mark.parametrize("off", [0, 8])  # elements of BF16: 0 and 16 bytes past a 32-byte boundary
+def test_forward_output_and_gate_alignment(off):
+    """The 32-byte and the 16-byte stores and gate loads give the same values."""
+    n, h, w = 2, 21, 37
+    X, Wt, b = case(n, h, w, 3)
+    Wk = Wt.permute(0, 2, 3, 1).reshape(32, 9, 32).contiguous()
+    size = n * h * w * 32
+    gate0 = torch.roll(X, 3, 3).contiguous()
+
+    def run(o):
+        buf = torch.full((size + 64,), 3.0, device="cuda:0", dtype=torch.bfloat16)
+        gb = torch.empty(size + 64, device="cuda:0", dtype=torch.bfloat16)
+        gb[o:o + size] = gate0.reshape(-1)
+        fb = torch.full((size + 64,), 3.0, device="cuda:0")
+        Y, g, Yf = buf[o:o + size], gb[o:o + size], fb[o // 2:o // 2 + size]
+        assert T.lib().tsu_corr_conv3x3(ptr(X), n, h, w, ptr(Wk), ptr(b), 1, ptr(g), ptr(Y), None, None) == 0
+        assert T.lib().tsu_corr_conv3x3(ptr(X), n, h, w, ptr(Wk), ptr(b), 0, None, None, ptr(Yf), None) == 0
+        assert T.lib().tsu_corr_status() == 0
+        assert bool((buf[:o] == 3.0).all()) and bool((buf[o + size:] == 3.0).all())
+        assert bool((fb[:o // 2] == 3.0).all()) and bool((fb[o // 2 + size:] == 3.0).all())
+        return Y.clone(), Yf.clone()
+
+    for a, c in zip(run(off), run(0)):
+        assert torch.equal(a, c)

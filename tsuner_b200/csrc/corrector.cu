@@ -70,12 +70,11 @@ constexpr int kChunks = 2;                   // chunk ring
 constexpr int kWBytes = 9 * 4 * 32 * 16;     // weights: 18432 B
 constexpr int kWBlk = 96 * 16;               // one (dx, channel quarter): 3 dy x 32 cout rows of 16 B
 constexpr int kAcc = 8;                      // TMEM accumulators (output rows) of 32 columns
-constexpr int kEpiWarps = 4;
+constexpr int kEpiWarps = 8;
 constexpr int kFwdCtas = 2;                  // CTAs per SM: one's issuing covers the other's
 constexpr int kFwdThreads = 64 + 32 * kEpiWarps;
-constexpr int kStage = kEpiWarps * 2048;
 constexpr int kFwdBars = (2 * kChunks + 2 * kAcc + 1) * 8 + 32;
-constexpr int kFwdSmem = 1024 + kWBytes + kChunks * kChunk + kStage + kFwdBars;
+constexpr int kFwdSmem = 1024 + kWBytes + kChunks * kChunk + kFwdBars;
 static_assert(kGrpBytes % 512 == 0 && kWBytes % 512 == 0, "swizzled TMA destinations");
 static_assert(kFwdCtas * (kFwdSmem + 1024) <= 228 * 1024 && kFwdCtas * 32 * kAcc <= 512, "residency");
 
@@ -212,6 +211,7 @@ struct ConvArgs {
     bf16 *Ybf;           // BF16 output, or
     float *Yf;           // FP32 output, or
     float *Y2;           // FP32 output of channels 0 and 1 only, [pixel][2] (the corrector's last layer)
+    int wide;            // output and gate lie on 32-byte boundaries
 };
 
 // A CTA's run of rows [b, e) of FwdGeom::rows, one segment (a range of rows of
@@ -233,96 +233,92 @@ struct Segments {
     }
 };
 
-// Epilogue of 32 pixels (4 groups of 8) of output row y: TMEM accumulators
+// 32 bytes of a pixel at once (the base 32-byte aligned), or as two halves
+__device__ __forceinline__ void store32(void *p, const uint32_t (&v)[8], bool wide) {
+    if (wide) {
+        asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+                     "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                     : "memory");
+    } else {
+        reinterpret_cast<uint4 *>(p)[0] = make_uint4(v[0], v[1], v[2], v[3]);
+        reinterpret_cast<uint4 *>(p)[1] = make_uint4(v[4], v[5], v[6], v[7]);
+    }
+}
+__device__ __forceinline__ void load32(const void *p, uint32_t (&v)[8], bool wide) {
+    if (wide) {
+        asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                     : "l"(p));
+    } else {
+        const uint4 a = __ldg(reinterpret_cast<const uint4 *>(p)), b = __ldg(reinterpret_cast<const uint4 *>(p) + 1);
+        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+    }
+}
+
+// Epilogue of 32 pixels (4 groups of 8) of an output row: TMEM accumulators
 // (lane = pixel, column = output channel) + bias, ReLU, optional gate, then
-// the store.  In NHWC a group's row is one contiguous run of 8 x 32 channels.
-// BF16 output (every layer but the last, and the input gradients) goes through
-// `sw` (2 KB of this warp): each lane writes its pixel's 4 x 16 B, then each
-// instruction stores one group's row as 32 lanes x 16 B contiguous.  16-byte
-// chunk k of pixel p sits in slot p * 4 + (k ^ ((p >> 1) & 3)), so both
-// patterns are free of bank conflicts.  FP32 output goes the same way in two
-// halves of 16 channels.  The gate is read per pixel.
-// px: element offset of this lane's own pixel at row 0 (-1: outside), row[r]:
-// of the pixel and chunk this lane stores of group r (-1: outside).
-__device__ __forceinline__ void conv_epilogue(const ConvArgs &a, int y, uint32_t taddr, int lane, const float *sBias,
-                                              uint4 *sw, const long long px, const long long (&row)[4],
-                                              uint64_t *release) {
-    const long long yo = (long long)y * a.W * C;
-    // the gate (4 x 16 B of this pixel; the lines stay in L1 across the 4
-    // loads) is requested before the TMEM read so the two latencies overlap
-    uint4 g[4];
+// the store of this lane's own pixel at element offset px (-1: outside the
+// image).  A pixel's channels are whole 32-byte sectors, so each lane stores
+// them itself, 32 bytes an instruction: staging them through shared memory
+// for contiguous 512-byte stores took twice the instructions and was what the
+// kernel waited for (8 x 528^2 with the gate: 95 us, now 78).
+__device__ __forceinline__ void conv_epilogue(const ConvArgs &a, uint32_t taddr, int lane, const float *sBias,
+                                              const long long px, uint64_t *release) {
+    // the gate is requested before the TMEM read so the two latencies overlap
+    uint32_t g[2][8];
     if (a.gate && px >= 0) {
-        const uint4 *gp = reinterpret_cast<const uint4 *>(a.gate + px + yo);
-#pragma unroll
-        for (int k = 0; k < 4; k++) g[k] = __ldg(gp + k);
+        load32(a.gate + px, g[0], a.wide);
+        load32(a.gate + px + 16, g[1], a.wide);
     }
     float acc[32];
     tmem_ld32(taddr, acc);
     fence_before();  // the accumulator is in registers: hand its TMEM columns back to the MMA issuer
     __syncwarp();
     if (lane == 0) mbar_arrive(release);
+    if (px < 0) return;
+    const float4 *b4 = reinterpret_cast<const float4 *>(sBias);
 #pragma unroll
-    for (int n = 0; n < 32; n++) {
-        float v = acc[n] + sBias[n];
-        if (a.relu) v = fmaxf(v, 0.f);
-        acc[n] = v;
+    for (int n = 0; n < 8; n++) {
+        const float4 b = b4[n];
+        acc[4 * n] += b.x;
+        acc[4 * n + 1] += b.y;
+        acc[4 * n + 2] += b.z;
+        acc[4 * n + 3] += b.w;
     }
-    if (a.gate && px >= 0) {
+    if (a.relu) {
+#pragma unroll
+        for (int n = 0; n < 32; n++) acc[n] = fmaxf(acc[n], 0.f);
+    }
+    if (a.gate) {
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162 *>(&g[k][j]);
+                if (!(__low2float(h) > 0.f)) acc[16 * k + 2 * j] = 0.f;
+                if (!(__high2float(h) > 0.f)) acc[16 * k + 2 * j + 1] = 0.f;
+            }
+        }
+    }
+    if (a.Y2) {  // the two used channels: 8 B per pixel
+        *reinterpret_cast<float2 *>(a.Y2 + px / C * 2) = make_float2(acc[0], acc[1]);
+    } else if (a.Yf) {
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            const uint32_t w[4] = {g[k].x, g[k].y, g[k].z, g[k].w};
+            uint32_t v[8];
 #pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const __nv_bfloat162 h = *reinterpret_cast<const __nv_bfloat162 *>(&w[j]);
-                if (!(__low2float(h) > 0.f)) acc[8 * k + 2 * j] = 0.f;
-                if (!(__high2float(h) > 0.f)) acc[8 * k + 2 * j + 1] = 0.f;
-            }
+            for (int j = 0; j < 8; j++) v[j] = __float_as_uint(acc[8 * k + j]);
+            store32(a.Yf + px + 8 * k, v, a.wide);
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            uint32_t v[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) v[j] = pack2(acc[16 * k + 2 * j], acc[16 * k + 2 * j + 1]);
+            store32(a.Ybf + px + 16 * k, v, a.wide);
         }
     }
-    const int rx = lane >> 2, kc = lane & 3;  // row phase: pixel of the group, 16-byte chunk
-    const int own = (lane >> 1) & 3;          // swizzle of this lane's own pixel
-    if (a.Y2) {  // the two used channels: 8 B per pixel, a group's row is 64 contiguous bytes
-        if (px >= 0) *reinterpret_cast<float2 *>(a.Y2 + (px + yo) / C * 2) = make_float2(acc[0], acc[1]);
-        return;
-    }
-    if (a.Yf) {  // FP32: two halves of 16 channels (64 B per pixel) through the same 2 KB
-#pragma unroll
-        for (int hf = 0; hf < 2; hf++) {
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const float *q = acc + 16 * hf + 4 * k;
-                sw[lane * 4 + (k ^ own)] = make_uint4(__float_as_uint(q[0]), __float_as_uint(q[1]),
-                                                      __float_as_uint(q[2]), __float_as_uint(q[3]));
-            }
-            __syncwarp();
-            uint4 v[4];
-#pragma unroll
-            for (int r = 0; r < 4; r++) {
-                const int p = r * 8 + rx;
-                v[r] = sw[p * 4 + (kc ^ ((p >> 1) & 3))];
-            }
-            __syncwarp();  // the next half overwrites the slots
-#pragma unroll
-            for (int r = 0; r < 4; r++)  // row[] counts 8 channels a chunk; here a chunk is 4
-                if (row[r] >= 0) *reinterpret_cast<uint4 *>(a.Yf + row[r] - kc * 4 + 16 * hf + yo) = v[r];
-        }
-        return;
-    }
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-        sw[lane * 4 + (k ^ own)] = make_uint4(pack2(acc[8 * k], acc[8 * k + 1]), pack2(acc[8 * k + 2], acc[8 * k + 3]),
-                                              pack2(acc[8 * k + 4], acc[8 * k + 5]), pack2(acc[8 * k + 6], acc[8 * k + 7]));
-    __syncwarp();
-    uint4 v[4];  // all four rows read before the first global store
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-        const int p = r * 8 + rx;
-        v[r] = sw[p * 4 + (kc ^ ((p >> 1) & 3))];
-    }
-    __syncwarp();  // the next row overwrites the slots
-#pragma unroll
-    for (int r = 0; r < 4; r++)
-        if (row[r] >= 0) *reinterpret_cast<uint4 *>(a.Ybf + row[r] + yo) = v[r];
 }
 
 // Forward convolution.  Persistent, two CTAs per SM; a CTA's rows come in
@@ -336,7 +332,7 @@ __device__ __forceinline__ void conv_epilogue(const ConvArgs &a, int y, uint32_t
 //     collects its taps in the order (dy, dx, half).  The first MMA of a row's
 //     first input overwrites (N = 32 of its own); at a segment's ends and
 //     where the ring wraps N is 32 or 64;
-//   warps 2-5: epilogue, a quarter of the row's pixels each.
+//   warps 2-9: epilogue, a quarter of the pixels of every other output row.
 // What bounded the one-tap form (18 MMAs of N = 32 per 128 pixels, the patch
 // as four 16-byte channel planes): each MMA reads 4 KB of A for 131 kFLOP, and
 // TMA writes 16 bytes at a time.  Here 6-7 MMAs read A once for three taps,
@@ -350,15 +346,14 @@ __global__ void __launch_bounds__(kFwdThreads, kFwdCtas)
     unsigned char *sm = smem_align<1024>(sm_raw);
     unsigned char *sW = sm;
     unsigned char *sP = sm + kWBytes;                  // chunk ring
-    unsigned char *sStage = sP + kChunks * kChunk;     // 2 KB per epilogue warp
-    uint64_t *full = reinterpret_cast<uint64_t *>(sStage + kStage);  // [kChunks] chunk landed
-    uint64_t *empty = full + kChunks;                                // [kChunks] chunk's MMAs done
-    uint64_t *accf = empty + kChunks;                                // [kAcc] accumulator ready
-    uint64_t *acce = accf + kAcc;                                    // [kAcc] accumulator read
-    uint64_t *fin = acce + kAcc;                                     // all MMAs done
+    uint64_t *full = reinterpret_cast<uint64_t *>(sP + kChunks * kChunk);  // [kChunks] chunk landed
+    uint64_t *empty = full + kChunks;                                      // [kChunks] chunk's MMAs done
+    uint64_t *accf = empty + kChunks;                                      // [kAcc] accumulator ready
+    uint64_t *acce = accf + kAcc;                                          // [kAcc] accumulator read
+    uint64_t *fin = acce + kAcc;                                           // all MMAs done
     uint32_t *tslot = reinterpret_cast<uint32_t *>(fin + 1);
     int *sCount = reinterpret_cast<int *>(tslot + 1);  // [0] chunks issued, [1] chunks waited for
-    __shared__ float sBias[32];
+    __shared__ __align__(16) float sBias[32];
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const FwdGeom G = fwd_geom(a.nimg, a.H, a.W);
 
@@ -504,22 +499,14 @@ __global__ void __launch_bounds__(kFwdThreads, kFwdCtas)
     } else {
         const int q = warp & 3;                  // TMEM lane quarter this warp may read
         const int par = (warp - 2) >> 2;         // output rows this warp takes: k % (kEpiWarps / 4)
-        uint4 *sw = reinterpret_cast<uint4 *>(sStage + (warp - 2) * 2048);
         int k = 0;
         bool ok = true;
         while (ok && seg.next()) {
-            // groups 4 q .. 4 q + 3 of the set: this lane's own pixel, and the
-            // pixel and chunk it stores of each
-            long long px = -1, row[4];
-#pragma unroll
-            for (int r = 0; r < 4; r++) {
-                const int g = seg.set * NG + 4 * q + r;
-                const int img = g / G.ntx, x0 = (g - img * G.ntx) * GX;
-                const long long o = (long long)img * a.H * a.W;
-                const int xr = x0 + (lane >> 2), xo = x0 + (lane & 7);
-                row[r] = (g < G.groups && xr < a.W) ? (o + xr) * C + (lane & 3) * 8 : -1;
-                if ((lane >> 3) == r && g < G.groups && xo < a.W) px = (o + xo) * C;
-            }
+            // this lane's pixel of groups 4 q .. 4 q + 3 of the set
+            const int g = seg.set * NG + 4 * q + (lane >> 3);
+            const int img = g / G.ntx, x = (g - img * G.ntx) * GX + (lane & 7);
+            const bool in = g < G.groups && x < a.W;
+            const long long p0 = ((long long)img * a.H * a.W + x) * C;
             for (int y = seg.y0; y < seg.y1; y++, k++) {
                 if (k % (kEpiWarps / 4) != par) continue;
                 const int ac = k % kAcc;
@@ -529,8 +516,8 @@ __global__ void __launch_bounds__(kFwdThreads, kFwdCtas)
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 fence_after();
-                conv_epilogue(a, y, tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(ac * 32), lane, sBias, sw, px, row,
-                              &acce[ac]);
+                conv_epilogue(a, tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(ac * 32), lane, sBias,
+                              in ? p0 + (long long)y * a.W * C : -1, &acce[ac]);
             }
         }
         if (!ok && lane == 0) atomicExch(&g_corr_err, 1);
@@ -997,10 +984,12 @@ int num_sms() {
     return n;
 }
 
-cudaError_t conv_launch(const ConvArgs &a, cudaStream_t st) {
+cudaError_t conv_launch(ConvArgs a, cudaStream_t st) {
     cudaError_t e = prepare();
     if (e != cudaSuccess) return e;
     if (reinterpret_cast<uintptr_t>(a.X) % 16) return cudaErrorInvalidValue;
+    a.wide = (reinterpret_cast<uintptr_t>(a.Ybf) | reinterpret_cast<uintptr_t>(a.Yf) |
+              reinterpret_cast<uintptr_t>(a.gate)) % 32 == 0;
     CUtensorMap mx;
     e = make_map(&mx, a.X, a.nimg, a.H, a.W, GW, kCRows);
     if (e != cudaSuccess) return e;
