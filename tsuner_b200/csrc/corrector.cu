@@ -768,7 +768,10 @@ __device__ __forceinline__ float up_bilinear(const float *__restrict__ p, int hc
     const int x1 = min(x0 + 1, wc - 1), y1 = min(y0 + 1, hc - 1);
     const float ax = fx - x0, ay = fy - y0;
     const float a = p[y0 * wc + x0], b = p[y0 * wc + x1], c = p[y1 * wc + x0], d = p[y1 * wc + x1];
-    return (1.f - ay) * ((1.f - ax) * a + ax * b) + ay * ((1.f - ax) * c + ax * d);
+    // the fused operations spelled out, so that the maps do not depend on what
+    // the compiler contracts in which kernel
+    const float lo = __fmaf_rn(ax, b, __fmul_rn(1.f - ax, a)), hi = __fmaf_rn(ax, d, __fmul_rn(1.f - ax, c));
+    return __fmaf_rn(1.f - ay, lo, __fmul_rn(ay, hi));
 }
 
 // The network runs on a canvas padded by kPad pixels on each side: a
@@ -796,42 +799,69 @@ __device__ __forceinline__ bool unpad(const Canvas &cv, int xp, int yp, int &x, 
 // coarse maps.
 //   coarse: [nsamples][3][hc*wc] = maximum depth, bed change, bathymetry H
 //   fineT:  [nsamples][2][H*W]   = maximum depth, bed change (or null)
-__global__ void features_kernel(const int *__restrict__ idx, int nb, const float *__restrict__ coarse,
-                                const float *__restrict__ fineT, const float *__restrict__ Hf, Canvas cv, int hc,
-                                int wc, int f, bf16 *__restrict__ X0, float *__restrict__ T, float *__restrict__ base) {
-    const long long npix = (long long)cv.H * cv.W, nppx = (long long)cv.Hp * cv.Wp;
-    for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < nb * nppx;
-         g += (long long)gridDim.x * blockDim.x) {
-        const int b = (int)(g / nppx);
-        const long long pp = g - (long long)b * nppx;
-        const int yp = (int)(pp / cv.Wp), xp = (int)(pp - (long long)yp * cv.Wp);
-        int x, y;
-        const bool inside = unpad(cv, xp, yp, x, y);
-        const long long p = (long long)y * cv.W + x;
-        const int s = idx[b];
-        const float *cs = coarse + (long long)s * 3 * hc * wc;
-        const float hm = up_bilinear(cs, hc, wc, f, x, y);
-        const float dbv = up_bilinear(cs + hc * wc, hc, wc, f, x, y);
-        const float Hc = up_bilinear(cs + 2 * hc * wc, hc, wc, f, x, y);
-        const float Hfine = Hf[p];
-        const int xi = min(x / f, wc - 1), yi = min(y / f, hc - 1);  // coarse cell containing the fine cell
-        const float wet = cs[yi * wc + xi] > 0.f ? 1.f : 0.f;
-        // channel 5 is 1 everywhere (a bias input); 6 and 7 locate the cell
-        // (the source enters through the west boundary)
-        const float v[8] = {hm / kSh, dbv / kSb, Hfine / kSH, (Hfine - Hc) / kSdH, wet, 1.f,
-                            (float)x / (float)max(cv.W - 1, 1), (float)y / (float)max(cv.H - 1, 1)};
-        uint4 *d = reinterpret_cast<uint4 *>(X0 + g * C);
-        d[0] = make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
-        d[1] = d[2] = d[3] = make_uint4(0, 0, 0, 0);
-        if (base) {
-            base[g * 2] = hm;
-            base[g * 2 + 1] = dbv;
+// A warp's unit is 32 consecutive pixels of a canvas row; their 64-byte records
+// are written as four runs of 512 contiguous bytes (chunk 0 of a pixel holds
+// its 8 features, the others are zeros).
+// 8 x 528^2: 62 -> 47 us, the loss below 44 -> 29 us (a pixel's 64 B per lane
+// and 64-bit divisions per pixel before).
+__device__ __forceinline__ void put_pixels32(bf16 *row, int xp0, int Wp, uint4 mine) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int from = i * 8 + (lane >> 2);
+        uint4 v;
+        v.x = __shfl_sync(0xffffffffu, mine.x, from);
+        v.y = __shfl_sync(0xffffffffu, mine.y, from);
+        v.z = __shfl_sync(0xffffffffu, mine.z, from);
+        v.w = __shfl_sync(0xffffffffu, mine.w, from);
+        if (lane & 3) v = make_uint4(0, 0, 0, 0);
+        if (xp0 + from < Wp) reinterpret_cast<uint4 *>(row + (size_t)(xp0 + from) * C)[lane & 3] = v;
+    }
+}
+// the units of nb canvases, one warp after another
+struct Units {
+    int segs, total;  // units per canvas row, units
+};
+__host__ __device__ inline Units units(const Canvas &cv, int nb) {
+    const int segs = (cv.Wp + 31) / 32;
+    return Units{segs, nb * cv.Hp * segs};
+}
+__global__ void __launch_bounds__(256)
+    features_kernel(const int *__restrict__ idx, int nb, const float *__restrict__ coarse, const float *__restrict__ fineT,
+                    const float *__restrict__ Hf, Canvas cv, int hc, int wc, int f, bf16 *__restrict__ X0,
+                    float *__restrict__ T, float *__restrict__ base) {
+    const long long npix = (long long)cv.H * cv.W;
+    const Units U = units(cv, nb);
+    for (int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < U.total; u += gridDim.x * blockDim.x >> 5) {
+        const int r = u / U.segs, b = r / cv.Hp, yp = r - b * cv.Hp;
+        const int xp = (u - r * U.segs) * 32 + (threadIdx.x & 31);
+        const long long row = (long long)r * cv.Wp;
+        uint4 mine = make_uint4(0, 0, 0, 0);
+        if (xp < cv.Wp) {
+            int x, y;
+            const bool inside = unpad(cv, xp, yp, x, y);
+            const long long p = (long long)y * cv.W + x;
+            const int s = idx[b];
+            const float *cs = coarse + (long long)s * 3 * hc * wc;
+            const float hm = up_bilinear(cs, hc, wc, f, x, y);
+            const float dbv = up_bilinear(cs + hc * wc, hc, wc, f, x, y);
+            const float Hc = up_bilinear(cs + 2 * hc * wc, hc, wc, f, x, y);
+            const float Hfine = Hf[p];
+            const int xi = min(x / f, wc - 1), yi = min(y / f, hc - 1);  // coarse cell containing the fine cell
+            const float wet = cs[yi * wc + xi] > 0.f ? 1.f : 0.f;
+            // channel 5 is 1 everywhere (a bias input); 6 and 7 locate the cell
+            // (the source enters through the west boundary)
+            const float v[8] = {hm / kSh, dbv / kSb, Hfine / kSH, (Hfine - Hc) / kSdH, wet, 1.f,
+                                (float)x / (float)max(cv.W - 1, 1), (float)y / (float)max(cv.H - 1, 1)};
+            mine = make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
+            if (base) reinterpret_cast<float2 *>(base)[row + xp] = make_float2(hm, dbv);
+            if (T && fineT) {
+                const float *ft = fineT + (long long)s * 2 * npix;
+                reinterpret_cast<float2 *>(T)[row + xp] =
+                    inside ? make_float2((ft[p] - hm) / kSh, (ft[npix + p] - dbv) / kSb) : make_float2(0.f, 0.f);
+            }
         }
-        if (T && fineT) {
-            const float *ft = fineT + (long long)s * 2 * npix;
-            T[g * 2] = inside ? (ft[p] - hm) / kSh : 0.f;
-            T[g * 2 + 1] = inside ? (ft[npix + p] - dbv) / kSb : 0.f;
-        }
+        put_pixels32(X0 + row * C, xp & ~31, cv.Wp, mine);
     }
 }
 
@@ -840,35 +870,35 @@ __global__ void features_kernel(const int *__restrict__ idx, int nb, const float
 // residual target), so that the few large residuals at run-up fronts weigh
 // more than their share of cells; dY = d(loss)/d(output) in BF16 (channels
 // 2..31 and the padding zero); loss sum accumulated in FP64.
-__global__ void loss_kernel(const float *__restrict__ Y, const float *__restrict__ T, int nb, Canvas cv, float wbig,
-                            bf16 *__restrict__ dY, double *__restrict__ loss) {
-    __shared__ double sred[32];
-    const long long nppx = (long long)cv.Hp * cv.Wp;
+__global__ void __launch_bounds__(256)
+    loss_kernel(const float *__restrict__ Y, const float *__restrict__ T, int nb, Canvas cv, float wbig,
+                bf16 *__restrict__ dY, double *__restrict__ loss) {
+    __shared__ double sred[8];
     const float scale = 1.f / (float)((long long)nb * cv.H * cv.W);  // d/dy of sum(w d^2) / (2 cells)
+    const Units U = units(cv, nb);
     double acc = 0.0;
-    for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < nb * nppx;
-         g += (long long)gridDim.x * blockDim.x) {
-        const long long pp = g % nppx;
-        const int yp = (int)(pp / cv.Wp), xp = (int)(pp - (long long)yp * cv.Wp);
+    for (int u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < U.total; u += gridDim.x * blockDim.x >> 5) {
+        const int r = u / U.segs, yp = r % cv.Hp;
+        const int xp = (u - r * U.segs) * 32 + (threadIdx.x & 31);
+        const long long row = (long long)r * cv.Wp;
+        uint4 mine = make_uint4(0, 0, 0, 0);
         int x, y;
-        float d0 = 0.f, d1 = 0.f, w0 = 0.f;
-        if (unpad(cv, xp, yp, x, y)) {
-            const float t0 = T[g * 2];
-            w0 = 1.f + wbig * t0 * t0;
-            d0 = Y[g * 2] - t0;
-            d1 = Y[g * 2 + 1] - T[g * 2 + 1];
+        if (xp < cv.Wp && unpad(cv, xp, yp, x, y)) {
+            const float2 t = reinterpret_cast<const float2 *>(T)[row + xp];
+            const float2 o = reinterpret_cast<const float2 *>(Y)[row + xp];
+            const float w0 = 1.f + wbig * t.x * t.x;
+            const float d0 = o.x - t.x, d1 = o.y - t.y;
             acc += (double)w0 * d0 * d0 + (double)d1 * d1;
+            mine.x = pack2(scale * w0 * d0, scale * d1);
         }
-        uint4 *gp = reinterpret_cast<uint4 *>(dY + g * C);
-        gp[0] = make_uint4(pack2(scale * w0 * d0, scale * d1), 0, 0, 0);
-        gp[1] = gp[2] = gp[3] = make_uint4(0, 0, 0, 0);
+        put_pixels32(dY + row * C, xp & ~31, cv.Wp, mine);
     }
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if ((threadIdx.x & 31) == 0) sred[threadIdx.x >> 5] = acc;
     __syncthreads();
     if (threadIdx.x == 0) {
         double s = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += sred[w];
+        for (int w = 0; w < 8; w++) s += sred[w];
         atomicAdd(loss, s);
     }
 }
@@ -1000,13 +1030,14 @@ cudaError_t conv_launch(ConvArgs a, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-// dW[k] += sum over CTAs of part[b][k]; db[n] += sum over CTAs and the 4 warps
-// of the bias partials.  A block owns 32 elements; each of its kRedWarps warps
+// dW[k] (+)= sum over CTAs of part[b][k]; db[n] (+)= sum over CTAs and the 4
+// warps of the bias partials; added to what is there, or in its place.  A block owns 32 elements; each of its kRedWarps warps
 // takes every kRedWarps-th row (all loads in flight together: the kernel is a
 // latency, not a bandwidth), then the sums are added in order.
 constexpr int kRedWarps = 16, kRedRows = 10;  // one pass covers 160 rows
-__global__ void __launch_bounds__(32 * kRedWarps) wgrad_reduce_kernel(const float *__restrict__ part, int nctas,
-                                                                      float *__restrict__ dW, float *__restrict__ db) {
+__global__ void __launch_bounds__(32 * kRedWarps)
+    wgrad_reduce_kernel(const float *__restrict__ part, int nctas, float *__restrict__ dW, float *__restrict__ db,
+                        bool add) {
     __shared__ float sSum[kRedWarps][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int k = blockIdx.x * 32 + lane;
@@ -1030,8 +1061,8 @@ __global__ void __launch_bounds__(32 * kRedWarps) wgrad_reduce_kernel(const floa
     if (w == 0) {
 #pragma unroll
         for (int q = 1; q < kRedWarps; q++) acc += sSum[q][lane];
-        if (!bias) dW[k] += acc;
-        else if (db) db[lane] += acc;
+        if (!bias) dW[k] = add ? dW[k] + acc : acc;
+        else if (db) db[lane] = add ? db[lane] + acc : acc;
     }
 }
 
@@ -1080,8 +1111,8 @@ void scratch_trim(int dev) {
 
 // part: wgrad_ctas(...) * kWgPart floats of device scratch, or null (then
 // allocated on the stream for this call)
-cudaError_t wgrad_launch(const bf16 *X, const bf16 *dZ, int nimg, int H, int W, float *dW, float *db, float *part,
-                         cudaStream_t st) {
+cudaError_t wgrad_launch(const bf16 *X, const bf16 *dZ, int nimg, int H, int W, float *dW, float *db, bool add,
+                         float *part, cudaStream_t st) {
     cudaError_t e = prepare();
     if (e != cudaSuccess) return e;
     if (reinterpret_cast<uintptr_t>(X) % 16 || reinterpret_cast<uintptr_t>(dZ) % 16) return cudaErrorInvalidValue;
@@ -1099,7 +1130,7 @@ cudaError_t wgrad_launch(const bf16 *X, const bf16 *dZ, int nimg, int H, int W, 
     conv3x3_wgrad_kernel<<<ctas, kWgThreads, kWgSmem, st>>>(mx, mz, nimg, H, W, part);
     e = cudaGetLastError();
     if (e == cudaSuccess) {
-        wgrad_reduce_kernel<<<KROWS + 1, 32 * kRedWarps, 0, st>>>(part, ctas, dW, db);
+        wgrad_reduce_kernel<<<KROWS + 1, 32 * kRedWarps, 0, st>>>(part, ctas, dW, db, add);
         e = cudaGetLastError();
     }
     if (own) {
@@ -1253,9 +1284,9 @@ int forward(TsuCorrector *c, int nb) {
 
 int load_batch(TsuCorrector *c, const int *idx, int nb, bool targets) {
     CCK(cudaMemcpyAsync(c->d_idx, idx, nb * sizeof(int), cudaMemcpyHostToDevice, c->st));
-    features_kernel<<<4 * num_sms(), 256, 0, c->st>>>(c->d_idx, nb, c->coarse, targets ? c->fine : nullptr, c->Hf, c->cv,
-                                                      c->hc, c->wc, c->f, c->act[0], targets ? c->T : nullptr,
-                                                      c->base);
+    features_kernel<<<8 * num_sms(), 256, 0, c->st>>>(c->d_idx, nb, c->coarse, targets ? c->fine : nullptr, c->Hf,
+                                                               c->cv, c->hc, c->wc, c->f, c->act[0],
+                                                               targets ? c->T : nullptr, c->base);
     CCK(cudaGetLastError());
     return TSU_OK;
 }
@@ -1455,15 +1486,13 @@ extern "C" int tsu_corr_train(TsuCorrector *c, int ntrain, int iters, int batch,
         if (rc) break;
         e = cudaMemsetAsync(c->d_loss, 0, 8, c->st);
         if (e != cudaSuccess) break;
-        loss_kernel<<<4 * num_sms(), 256, 0, c->st>>>(c->Yout, c->T, batch, c->cv, c->wbig, c->g0, c->d_loss);
+        loss_kernel<<<8 * num_sms(), 256, 0, c->st>>>(c->Yout, c->T, batch, c->cv, c->wbig, c->g0, c->d_loss);
         if ((e = cudaGetLastError()) != cudaSuccess) break;
         if ((e = cudaMemcpyAsync(h_loss + it, c->d_loss, 8, cudaMemcpyDeviceToHost, c->st)) != cudaSuccess) break;
-        if ((e = cudaMemsetAsync(c->gW, 0, nw * 4, c->st)) != cudaSuccess) break;
-        if ((e = cudaMemsetAsync(c->gB, 0, (size_t)L * 32 * 4, c->st)) != cudaSuccess) break;
         bf16 *dZ = c->g0, *dX = c->g1;
         for (int l = L - 1; l >= 0 && e == cudaSuccess; l--) {
             e = wgrad_launch(c->act[l], dZ, batch, c->cv.Hp, c->cv.Wp, c->gW + (size_t)l * 32 * KROWS, c->gB + l * 32,
-                             c->wg_part, c->st);
+                             false, c->wg_part, c->st);
             if (e == cudaSuccess && l > 0) {  // dZ_{l-1} = conv(dZ_l, flipped W_l), zero where act[l] <= 0
                 ConvArgs a;
                 a.X = dZ;
@@ -1617,7 +1646,7 @@ extern "C" int tsu_corr_conv3x3(const void *X, int nimg, int H, int W, const voi
 extern "C" int tsu_corr_conv3x3_wgrad(const void *X, const void *dZ, int nimg, int H, int W, float *dW, float *db,
                                       void *stream) {
     if (!X || !dZ || !dW || nimg < 1 || H < 1 || W < 1) return TSU_ERR_INVALID;
-    CCK(wgrad_launch(static_cast<const bf16 *>(X), static_cast<const bf16 *>(dZ), nimg, H, W, dW, db, nullptr,
+    CCK(wgrad_launch(static_cast<const bf16 *>(X), static_cast<const bf16 *>(dZ), nimg, H, W, dW, db, true, nullptr,
                      static_cast<cudaStream_t>(stream)));
     return TSU_OK;
 }
