@@ -934,6 +934,23 @@ __global__ void adam_kernel(float *__restrict__ Wm, float *__restrict__ mW, floa
     }
 }
 
+// The BF16 weights and their tap-flipped transpose (as adam_kernel refreshes
+// them) from new master weights, and Adam's moments to zero.
+__global__ void load_weights_kernel(const float *__restrict__ Wm, int nlayers, bf16 *__restrict__ Wbf,
+                                    bf16 *__restrict__ Wt, float *__restrict__ mW, float *__restrict__ vW,
+                                    float *__restrict__ mB, float *__restrict__ vB) {
+    const int nw = nlayers * 32 * KROWS;
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nw; k += gridDim.x * blockDim.x) {
+        const int l = k / (32 * KROWS), r = k - l * 32 * KROWS, co = r / KROWS, kk = r - co * KROWS;
+        const int tap = kk / 32, ci = kk - tap * 32;
+        const bf16 w = __float2bfloat16_rn(Wm[k]);
+        Wbf[k] = w;
+        Wt[l * 32 * KROWS + ci * KROWS + (8 - tap) * 32 + co] = w;
+        mW[k] = vW[k] = 0.f;
+        if (k < nlayers * 32) mB[k] = vB[k] = 0.f;
+    }
+}
+
 // Per-cell envelope of the training targets: E[c][p] = max over the batch
 // (and earlier batches) of |T[b][p][c]| over the fine cells p.  Non-negative
 // floats order like their bit patterns, so the maximum is an integer
@@ -1185,6 +1202,13 @@ struct TsuCorrector {
     float *E = nullptr;
     int env_n = 0, ntrain = 0;
     float *wg_part = nullptr;  // weight-gradient partials of one layer ([CTAs][kWgPart])
+    // predictions: two maps of one sample each ([4][H*W]), so that one is copied
+    // to the host (on cp) while the next is computed; made at the first prediction
+    float *out[2] = {};
+    cudaStream_t cp = nullptr;
+    cudaEvent_t done[2] = {};
+    double *h_loss = nullptr;  // pinned, one per training iteration, grown when needed
+    int h_loss_cap = 0;
 };
 
 namespace {
@@ -1208,8 +1232,12 @@ double uniform01(uint64_t &s) { return (double)(splitmix(s) >> 11) * (1.0 / 9007
 
 void free_all(TsuCorrector *c) {
     float *fp[] = {c->Wm, c->mW, c->vW, c->gW, c->Bm, c->mB, c->vB, c->gB, c->Yout, c->T, c->base, c->Hf, c->coarse, c->fine,
-                   c->E, c->wg_part};
+                   c->E, c->wg_part, c->out[0], c->out[1]};
     for (float *p : fp) cudaFree(p);
+    if (c->h_loss) cudaFreeHost(c->h_loss);
+    for (cudaEvent_t ev : c->done)
+        if (ev) cudaEventDestroy(ev);
+    if (c->cp) cudaStreamDestroy(c->cp);
     cudaFree(c->Wbf);
     cudaFree(c->Wt);
     for (bf16 *p : c->act) cudaFree(p);
@@ -1225,24 +1253,10 @@ void free_all(TsuCorrector *c) {
 int upload_weights(TsuCorrector *c, const float *W, const float *B) {
     const int L = TsuCorrector::L;
     const size_t nw = (size_t)L * 32 * KROWS;
-    std::vector<bf16> wb(nw), wt(nw);
-    for (int l = 0; l < L; l++)
-        for (int co = 0; co < 32; co++)
-            for (int kk = 0; kk < KROWS; kk++) {
-                const size_t k = ((size_t)l * 32 + co) * KROWS + kk;
-                const int tap = kk / 32, ci = kk % 32;
-                const bf16 v = __float2bfloat16_rn(W[k]);
-                wb[k] = v;
-                wt[(size_t)l * 32 * KROWS + ci * KROWS + (8 - tap) * 32 + co] = v;
-            }
     CCK(cudaMemcpyAsync(c->Wm, W, nw * sizeof(float), cudaMemcpyHostToDevice, c->st));
     CCK(cudaMemcpyAsync(c->Bm, B, (size_t)L * 32 * sizeof(float), cudaMemcpyHostToDevice, c->st));
-    CCK(cudaMemcpyAsync(c->Wbf, wb.data(), nw * sizeof(bf16), cudaMemcpyHostToDevice, c->st));
-    CCK(cudaMemcpyAsync(c->Wt, wt.data(), nw * sizeof(bf16), cudaMemcpyHostToDevice, c->st));
-    CCK(cudaMemsetAsync(c->mW, 0, nw * sizeof(float), c->st));
-    CCK(cudaMemsetAsync(c->vW, 0, nw * sizeof(float), c->st));
-    CCK(cudaMemsetAsync(c->mB, 0, (size_t)L * 32 * sizeof(float), c->st));
-    CCK(cudaMemsetAsync(c->vB, 0, (size_t)L * 32 * sizeof(float), c->st));
+    load_weights_kernel<<<(int)((nw + 255) / 256), 256, 0, c->st>>>(c->Wm, L, c->Wbf, c->Wt, c->mW, c->vW, c->mB, c->vB);
+    CCK(cudaGetLastError());
     CCK(cudaStreamSynchronize(c->st));
     c->adam_t = 0;
     return TSU_OK;
@@ -1475,8 +1489,14 @@ extern "C" int tsu_corr_train(TsuCorrector *c, int ntrain, int iters, int batch,
     const long long npix = (long long)batch * c->H * c->W;
     uint64_t s = seed;
     std::vector<int> idx(batch);
-    double *h_loss = nullptr;
-    CCK(cudaMallocHost((void **)&h_loss, sizeof(double) * std::max(iters, 1)));
+    if (iters > c->h_loss_cap) {  // kept between calls: page-locking memory costs more than an iteration
+        if (c->h_loss) cudaFreeHost(c->h_loss);
+        c->h_loss = nullptr;
+        c->h_loss_cap = 0;
+        CCK(cudaMallocHost((void **)&c->h_loss, sizeof(double) * iters));
+        c->h_loss_cap = iters;
+    }
+    double *const h_loss = c->h_loss;
     int rc = TSU_OK;
     cudaError_t e = cudaEventRecord(c->e0, c->st);
     for (int it = 0; it < iters && !rc && e == cudaSuccess; it++) {
@@ -1532,7 +1552,6 @@ extern "C" int tsu_corr_train(TsuCorrector *c, int ntrain, int iters, int batch,
         if (loss)
             for (int it = 0; it < iters; it++) loss[it] = (float)(h_loss[it] / (2.0 * (double)npix));
     }
-    cudaFreeHost(h_loss);
     if (rc) return rc;
     return check_kernel_flag();
 }
@@ -1550,16 +1569,29 @@ extern "C" int tsu_corr_predict(TsuCorrector *c, int first, int n, float *out_hm
         const int r = compute_envelope(c, c->ntrain);
         if (r) return r;
     }
-    float *d_out = nullptr;
-    CCK(cudaMalloc((void **)&d_out, 4 * np * 4));
-    int rc = TSU_OK;
-    for (int k = 0; k < n && !rc; k++) {
+    if (!c->cp) {
+        for (int q = 0; q < 2; q++) {
+            if (!c->out[q]) CCK(cudaMalloc((void **)&c->out[q], 4 * np * 4));
+            if (!c->done[q]) CCK(cudaEventCreateWithFlags(&c->done[q], cudaEventDisableTiming));
+        }
+        CCK(cudaStreamCreateWithFlags(&c->cp, cudaStreamNonBlocking));
+    }
+    auto compute = [&](int k) -> int {  // sample first + k -> out[k & 1]
         const int s = first + k;
-        rc = load_batch(c, &s, 1, false);
-        if (!rc) rc = forward(c, 1);
-        if (rc) break;
+        int r = load_batch(c, &s, 1, false);
+        if (!r) r = forward(c, 1);
+        if (r) return r;
         apply_kernel<<<2 * num_sms(), 256, 0, c->st>>>(c->Yout, c->base, c->cv, c->clip_depth, clamp ? c->E : nullptr,
-                                                         c->envelope, d_out);
+                                                         c->envelope, c->out[k & 1]);
+        CCK(cudaGetLastError());
+        CCK(cudaEventRecord(c->done[k & 1], c->st));
+        return TSU_OK;
+    };
+    int rc = compute(0);
+    for (int k = 0; k < n && !rc; k++) {
+        // the other map's copy (of sample k - 1) has ended: planes_d2h waits for it
+        if (k + 1 < n) rc = compute(k + 1);
+        if (rc) break;
         float *want[4] = {out_hmax, out_db, base_hmax, base_db};
         void *outs[4];
         const void *ins[4];
@@ -1567,17 +1599,20 @@ extern "C" int tsu_corr_predict(TsuCorrector *c, int first, int n, float *out_hm
         for (int q = 0; q < 4; q++)
             if (want[q]) {
                 outs[m] = want[q] + k * np;
-                ins[m++] = d_out + q * np;
+                ins[m++] = c->out[k & 1] + q * np;
             }
-        if (cudaGetLastError() != cudaSuccess ||
-            tsu::planes_d2h(m, outs, (size_t)c->W * 4, ins, (size_t)c->W * 4, (size_t)c->W * 4, c->H, c->st) != cudaSuccess ||
-            cudaStreamSynchronize(c->st) != cudaSuccess) {
+        if (cudaStreamWaitEvent(c->cp, c->done[k & 1], 0) != cudaSuccess ||
+            tsu::planes_d2h(m, outs, (size_t)c->W * 4, ins, (size_t)c->W * 4, (size_t)c->W * 4, c->H, c->cp) != cudaSuccess ||
+            cudaStreamSynchronize(c->cp) != cudaSuccess) {
             snprintf(g_corr_msg, sizeof(g_corr_msg), "tsu_corr_predict: CUDA error");
             rc = TSU_ERR_CUDA;
             break;
         }
     }
-    cudaFree(d_out);
+    if (cudaStreamSynchronize(c->st) != cudaSuccess && !rc) {
+        snprintf(g_corr_msg, sizeof(g_corr_msg), "tsu_corr_predict: CUDA error");
+        rc = TSU_ERR_CUDA;
+    }
     if (rc) return rc;
     return check_kernel_flag();
 }
