@@ -146,6 +146,30 @@ __device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, i
         : "memory");
 }
 
+// Programmatic dependent launch: a kernel launched with launch_after() may
+// start while the kernel before it on the stream is still running its last
+// CTAs.  prior_grids_done() returns once that kernel has completed and its
+// writes are visible; nothing it wrote, and nothing it may still read, is
+// touched before.  next_grid_may_start() lets the kernel after this one take
+// the SM slots that this one's CTAs leave.
+__device__ __forceinline__ void prior_grids_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void next_grid_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+cudaError_t launch_after(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, static_cast<A &&>(args)...);
+}
+
 // host: cuTensorMapEncodeTiled from the driver (no link against libcuda)
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,

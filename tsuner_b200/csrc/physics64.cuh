@@ -216,22 +216,24 @@ __device__ __forceinline__ Face5 filter_face(double &h, double &qx, double &qy, 
         return face_of<false>(h, qx, qy, H, hc, ok);
     }
     bool in = true;
-    const Divisor<true> d(h + kEpsilon, in);
+    Divisor<true> d(h + kEpsilon, in);
+    // without water: a zero reciprocal makes every quotient below a zero
+    const bool dry = (h == 0.0) & (hc == 0.0) & (fabs(qx) + fabs(qy) < 1e30);
+    d.y = dry ? 0.0 : d.y;
     double c = d.of(hc, in);
     const double u = d.of(qx), v = d.of(qy);
     in &= wet_divisor(d.d) & calm(qx, u) & calm(qy, v);
-    const bool dry = (h == 0.0) & (hc == 0.0) & (fabs(qx) + fabs(qy) < 1e30);
     ok &= in | dry;
     c = (c > 0.0) ? c : 0.0;
-    qx = dry ? 0.0 : h * u;
-    qy = dry ? 0.0 : h * v;
+    qx = h * u;
+    qy = h * v;
     hc = h * c;
     Face5 f;
     f.h = h;
     f.H = H;
-    f.u = dry ? 0.0 : d.near(qx, u);
-    f.v = dry ? 0.0 : d.near(qy, v);
-    f.c = dry ? 0.0 : d.near(hc, c);
+    f.u = d.near(qx, u);
+    f.v = d.near(qy, v);
+    f.c = d.near(hc, c);
     return f;
 }
 
@@ -243,9 +245,11 @@ __device__ __forceinline__ double limit(double a, double b, bool &ok) {
     if (!FAST) return limiter(a, b);
     const double p = a * b, s = a + b;
     const bool live = (p > 0.0) & (fabs(s) > kEpsilon);
-    const Divisor<true> d(live ? s : 1.0, ok);
-    ok &= mid(p) | !live;
-    return d.of(live ? p + p : 0.0);
+    bool in = mid(p);
+    const Divisor<true> d(s, in);
+    const double q = d.of(p + p);
+    ok &= in | !live;  // else q is not used
+    return live ? q : 0.0;
 }
 
 // bedload (GPU/SedFlux.cuh:150-168), or the Grass law when selected; modu
@@ -309,17 +313,7 @@ __device__ __forceinline__ bool edge_flux(const Phys64 &P, const Face5 &a, const
         for (int i = 0; i < 5; i++) Dm[i] = Dp[i] = z;
         return true;
     }
-    double F0[5], F1[5];
-    // bed fluxes first: the only part with a branch
-    F0[3] = F1[3] = 0.0;
-    const bool moves = (fixed != 0) & (P.bedload != 0);
-    if (!FAST || (moves & (P.bedload_law != 0))) {
-        F0[3] = bed_flux(P, h0, a.u, a.v, moves);
-        F1[3] = bed_flux(P, h1, b.u, b.v, moves);
-    } else if (moves & !(P.still(a.u) & P.still(a.v) & P.still(b.u) & P.still(b.v))) {
-        F0[3] = bed_flux_fast(P, h0, a.u, a.v, ok);
-        F1[3] = bed_flux_fast(P, h1, b.u, b.v, ok);
-    }
+    double F0[5], F1[5];  // [3], the bed, comes last
     const double hc0 = h0 * a.c, hc1 = h1 * b.c;
     F0[0] = h0 * a.u;
     F0[1] = F0[0] * a.u;
@@ -359,24 +353,40 @@ __device__ __forceinline__ bool edge_flux(const Phys64 &P, const Face5 &a, const
     }
 
     double df[5], DU[5];
-#pragma unroll
-    for (int i = 0; i < 5; i++) df[i] = F1[i] - F0[i];
-    df[1] += ghm * deta;
+    df[0] = F1[0] - F0[0];
+    df[1] = (F1[1] - F0[1]) + ghm * deta;
+    df[2] = F1[2] - F0[2];
+    df[4] = F1[4] - F0[4];
     DU[0] = deta;
-    DU[1] = F1[0] - F0[0];  // q = u h, the mass flux
+    DU[1] = df[0];  // q = u h, the mass flux
     DU[2] = b.v * h1 - a.v * h0;
-    DU[3] = 0.0;  // replaced by the upwinded bed component below
     DU[4] = hc1 - hc0;
-    const int s0 = sgn(b.H - a.H), s2 = sgn(a1);
-    const int s1 = sgn(df[3]) * s0;  // s1 / s0 for s0 = +-1, 0 for s0 = 0
-    double vis[5];
-#pragma unroll
-    for (int i = 0; i < 5; i++) vis[i] = a0 * DU[i] + a1 * df[i];
-    vis[3] = (s2 == s1) ? a1 * df[3] : -a1 * df[3];
 #pragma unroll
     for (int i = 0; i < 5; i++) {
-        Dm[i] = 0.5 * (df[i] - vis[i]) + F0[i];
-        Dp[i] = 0.5 * (df[i] + vis[i]) - F1[i];
+        if (i == 3) continue;
+        const double vis = a0 * DU[i] + a1 * df[i];
+        Dm[i] = 0.5 * (df[i] - vis) + F0[i];
+        Dp[i] = 0.5 * (df[i] + vis) - F1[i];
+    }
+    // the bed component (upwinded by its own sign, :100-120): zeros where the
+    // bed is fixed or at rest on both sides
+    const bool moves = (fixed != 0) & (P.bedload != 0);
+    Dm[3] = Dp[3] = 0.0;
+    if (!FAST || (moves & ((P.bedload_law != 0) | !(P.still(a.u) & P.still(a.v) & P.still(b.u) & P.still(b.v))))) {
+        double f0, f1;
+        if (!FAST || P.bedload_law != 0) {
+            f0 = bed_flux(P, h0, a.u, a.v, moves);
+            f1 = bed_flux(P, h1, b.u, b.v, moves);
+        } else {
+            f0 = bed_flux_fast(P, h0, a.u, a.v, ok);
+            f1 = bed_flux_fast(P, h1, b.u, b.v, ok);
+        }
+        const double d = f1 - f0;
+        const int s0 = sgn(b.H - a.H), s2 = sgn(a1);
+        const int s1 = sgn(d) * s0;  // s1 / s0 for s0 = +-1, 0 for s0 = 0
+        const double vis = (s2 == s1) ? a1 * d : -a1 * d;
+        Dm[3] = 0.5 * (d - vis) + f0;
+        Dp[3] = 0.5 * (d + vis) - f1;
     }
     return ok;
 }

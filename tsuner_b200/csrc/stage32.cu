@@ -165,10 +165,6 @@ __device__ __forceinline__ void stage32_tile(const Stage32Args &A, const Phys32 
     // Global memory is accessed through explicit global-space loads and
     // stores: in the ensemble the buffer pointers come from a descriptor in
     // shared memory, and generic accesses through them are slower.
-    const double t = __ldcg(A.scal + SC_T);
-    if (!(t < __ldcg(A.scal + SC_TEND))) return;  // run_until predicate (uniform per grid)
-    const double dtd = __ldcg(A.scal + SC_DT);
-    const float dt = (float)dtd;
     const int npx = P.npx, npy = P.npy;
     const bool periodic = (P.wbc == 2);
     const int tid = threadIdx.x;
@@ -239,6 +235,9 @@ __device__ __forceinline__ void stage32_tile(const Stage32Args &A, const Phys32 
         prefetch_l2(A.bmin + gown);
         prefetch_l2(A.eta_max + gown);
     }
+    // the scalars are read while the box travels
+    const double t = __ldcg(A.scal + SC_T), tend = __ldcg(A.scal + SC_TEND), dtd = __ldcg(A.scal + SC_DT);
+    const float dt = (float)dtd;
     __syncthreads();
     if (use_tma) {  // every thread sees the box land (bounded wait)
         const bool ok = mbar_wait_first(&sBar, 0);
@@ -250,6 +249,7 @@ __device__ __forceinline__ void stage32_tile(const Stage32Args &A, const Phys32 
             return;
         }
     }
+    if (!(t < tend)) return;  // run_until predicate (uniform per grid)
     const int cidx = (ty + 2) * LX + (tx + HX);
     float vc[5];
 #pragma unroll
@@ -694,6 +694,8 @@ template <int TX, int TY, int MINB, int ORDER, bool FIRST, bool LAST>
 __global__ void __launch_bounds__(TX *TY, MINB)
     stage32_kernel(const __grid_constant__ Stage32Args A, const __grid_constant__ Tma32 M) {
     extern __shared__ __align__(16) float smem32[];
+    prior_grids_done();
+    next_grid_may_start();
     stage32_tile<TX, TY, ORDER, FIRST, LAST>(A, A.phys, &M, blockIdx.x, blockIdx.y,
                                              blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y, smem32);
 }
@@ -711,6 +713,8 @@ __global__ void __launch_bounds__(TX *TY, MINB) ens32_kernel(EnsArgs E, Phys32 c
     extern __shared__ __align__(16) float smem32[];
     __shared__ Stage32Args sG;
     __shared__ unsigned sTile;
+    prior_grids_done();
+    next_grid_may_start();
     unsigned tile = blockIdx.x;
     if (E.dynamic) {
         if (threadIdx.x == 0) sTile = atomicAdd(E.work, 1u);
@@ -992,16 +996,14 @@ dim3 stage32_grid(int npx, int npy) {
 cudaError_t stage32_launch(int order, int stage, const Stage32Args &a, const Tma32 &tm, cudaStream_t st) {
     const Variant32 &v = variants32(nullptr)[single_variant()];
     dim3 g = stage32_grid(a.phys.npx, a.phys.npy);
-    v.k[which(order, stage)]<<<g, v.tx * v.ty, v.smem, st>>>(a, tm);
-    return cudaGetLastError();
+    return launch_after(v.k[which(order, stage)], g, dim3(v.tx * v.ty), v.smem, st, a, tm);
 }
 
 cudaError_t ens32_launch(int variant, int order, int stage, const EnsArgs &e, const Phys32 &common, int ctas,
                          cudaStream_t st) {
     const Variant32 &v = variants32(nullptr)[variant];
     if (e.dynamic) reset_work_kernel<<<1, 1, 0, st>>>(e.work);
-    v.e[which(order, stage)]<<<ctas, v.tx * v.ty, v.smem, st>>>(e, common);
-    return cudaGetLastError();
+    return launch_after(v.e[which(order, stage)], dim3(ctas), dim3(v.tx * v.ty), v.smem, st, e, common);
 }
 
 int ens32_max_ctas_per_sm(int variant) {

@@ -308,15 +308,19 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
     unsigned char *sM = reinterpret_cast<unsigned char *>(smem) + T::kMaskOff;  // [LY][MLX], tile at column MHX
     __shared__ int sLast;
 
-    const double t = A.scal[SC_T];
-    if (!(t < A.scal[SC_TEND])) return;  // run_until predicate (uniform)
-    const double dt = A.scal[SC_DT];
-
     const int npx = P.npx, npy = P.npy;
     const bool periodic = (P.wbc == 2);
     const int tid = threadIdx.x;
     const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
     const long long pitch = A.pitch, plane = A.plane;
+
+    if (threadIdx.x == 0) {  // barriers of the tile's loads, before anything the previous kernel may still hold up
+        mbar_init(&sBar, 1);
+        if (OWN == 2 && !FIRST) mbar_init(&sBarOwn, 1);
+        mbar_init_fence();
+    }
+    prior_grids_done();
+    next_grid_may_start();
 
     const double *Vin;
     const double *V0;
@@ -351,9 +355,6 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
     double *sOwn = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(smem) + T::kOwnOff);
     if (use_tma) {
         if (tid == 0) {
-            mbar_init(&sBar, 1);
-            if (own_tma) mbar_init(&sBarOwn, 1);
-            mbar_init_fence();
             mbar_expect_tx(&sBar, 5 * PS * sizeof(double) + T::MPS);
             // the tensor maps start at the first stored row (a slab's lowest ghost row)
             tma_load_3d(sV, (Vin == A.bufB) ? &A.tmB : &A.tmA, x0 - 2, y0 - 2 + P.gs, 0, &sBar);
@@ -401,6 +402,8 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
         prefetch_l2(A.bmin + gown);
         prefetch_l2(A.eta_max + gown);
     }
+    // the scalars are read while the boxes travel
+    const double t = A.scal[SC_T], tend = A.scal[SC_TEND], dt = A.scal[SC_DT];
     __syncthreads();
     if (use_tma) {  // every thread sees the box land (bounded wait)
         const bool ok = mbar_wait_first(&sBar, 0);
@@ -412,6 +415,11 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
             }
             return;
         }
+    }
+
+    if (!(t < tend)) {  // run_until predicate (uniform); the other boxes land first
+        if (own_tma && tid == 0) mbar_wait(&sBarOwn, 0);
+        return;
     }
 
     const int cidx = (ty + 2) * LX + (tx + 2);
@@ -1114,8 +1122,7 @@ cudaError_t stage64_launch(int order, int stage, const Stage64Args &a, cudaStrea
     dim3 g = stage64_grid(a.phys.npx, a.phys.npy);
     int which = (order == 2) ? (stage == 0 ? 0 : 1) : 2;
     if (a.phys.rk == 0) which = (order == 2) ? 3 : 4;  // MUSCL-Hancock: one stage
-    v.k[which]<<<g, v.nthr, v.smem, st>>>(a);
-    return cudaGetLastError();
+    return launch_after(v.k[which], g, dim3(v.nthr), v.smem, st, a);
 }
 
 cudaError_t initial_dt_launch(const double *V, long long pitch, long long plane, const Phys64 &P, double *partials,
