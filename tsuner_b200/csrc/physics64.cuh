@@ -185,18 +185,23 @@ __device__ __forceinline__ bool calm(double q, double u) {
 }
 static_assert(kVmax == 10.0 && kEps < 0x1p-19, "calm, wet_divisor");
 
+// dry land: a state of zeros
+__device__ __forceinline__ bool empty(double h, double qx, double qy, double hc) {
+    return ((hi32(h) | hi32(qx) | hi32(qy) | hi32(hc)) << 1 | lo32(h) | lo32(qx) | lo32(qy) | lo32(hc)) == 0u;
+}
+
 // Velocity and concentration of an unfiltered state (a cell, a ghost).
 template <bool FAST>
 __device__ __forceinline__ Face5 face_of(double h, double qx, double qy, double H, double hc, bool &ok) {
     Face5 f;
     f.h = h;
     f.H = H;
-    if (FAST) {
+    if (FAST) {  // wet and unclamped, or empty (zero over EPSILON throughout)
         const Divisor<true> d(h + kEpsilon, ok);
         f.u = d.of(qx);
         f.v = d.of(qy);
         f.c = d.of(hc, ok);
-        ok &= wet_divisor(d.d) & calm(qx, f.u) & calm(qy, f.v);
+        ok &= (wet_divisor(d.d) & calm(qx, f.u) & calm(qy, f.v)) | empty(h, qx, qy, hc);
     } else {
         velocity(h, qx, qy, f.u, f.v);
         f.c = ddiv(hc, h + kEpsilon);
@@ -207,8 +212,8 @@ __device__ __forceinline__ Face5 face_of(double h, double qx, double qy, double 
 // A state through the positivity filter (state_filter_double,
 // GPU/SedFlux.cuh:118-132), and the velocity and concentration of the result;
 // h, qx, qy, hc become the filtered ones.  FAST: a wet, unclamped state (six
-// quotients by the same h + EPSILON) or one without water and load, which
-// comes out as zeros; `dry` says which.
+// quotients by the same h + EPSILON) or one without water, which comes out as
+// zeros.
 template <bool FAST>
 __device__ __forceinline__ Face5 filter_face(double &h, double &qx, double &qy, double H, double &hc, bool &ok) {
     if (!FAST) {
@@ -218,7 +223,7 @@ __device__ __forceinline__ Face5 filter_face(double &h, double &qx, double &qy, 
     bool in = true;
     Divisor<true> d(h + kEpsilon, in);
     // without water: a zero reciprocal makes every quotient below a zero
-    const bool dry = (h == 0.0) & (hc == 0.0) & (fabs(qx) + fabs(qy) < 1e30);
+    const bool dry = (h == 0.0) & (fabs(qx) + fabs(qy) + fabs(hc) < 1e30);
     d.y = dry ? 0.0 : d.y;
     double c = d.of(hc, in);
     const double u = d.of(qx), v = d.of(qy);
@@ -498,11 +503,15 @@ __device__ __forceinline__ double cfl_dt(const Phys64 &P, double h, double qx, d
     return P.CFL * 0.5 * fmin(ddiv_inf(P.dx, lx), ddiv_inf(P.dy, ly));
 }
 
-// The same of a wet cell from the velocity of its filtered state.  On square
+// The same from the velocity of the cell's filtered state.  On square
 // cells the smaller of dx / lx and dy / ly is dx over the larger speed (the
 // rounded quotient does not increase with the divisor).
 __device__ __forceinline__ bool cfl_dt_fast(const Phys64 &P, const Face5 &f, double &dt) {
     bool ok = mid(f.h);
+    if (f.h == 0.0) {  // no speed: an infinite step
+        dt = CUDART_INF;
+        return true;
+    }
     const double cg = root(kG * f.h);
     const double lx = fabs(f.u) + cg, ly = fabs(f.v) + cg;
     double q;

@@ -224,7 +224,9 @@ __device__ __forceinline__ bool sources(const Phys64 &P, double dt, const double
         ux = d0.of(v0[1]);
         uy = d0.of(v0[2]);
         const double m2 = ux * ux + uy * uy;
-        ok &= wet_divisor(d0.d) & calm(v0[1], ux) & calm(v0[2], uy) & mid_or_zero(m2);
+        // an empty cell: every quotient by EPSILON or eps_h is a zero
+        ok &= (wet_divisor(d0.d) & calm(v0[1], ux) & calm(v0[2], uy) & mid_or_zero(m2)) |
+              (empty(v0[0], v0[1], v0[2], v0[4]) & mid(P.eps_h));
         modu = root(m2);
     } else {
         velocity(v0[0], v0[1], v0[2], ux, uy);
@@ -434,9 +436,8 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
     // ---- phase 2: per-cell velocity and concentration
     for (int idx = tid; idx < PS; idx += NT) {
         const double h = sV[idx], qx = sV[PS + idx], qy = sV[2 * PS + idx], hc = sV[4 * PS + idx];
-        bool ok = wet_divisor(h);
-        Face5 f;
-        if (ok) f = face_of<true>(h, qx, qy, 0.0, hc, ok);
+        bool ok = true;
+        Face5 f = face_of<true>(h, qx, qy, 0.0, hc, ok);
         if (!ok) f = face_of<false>(h, qx, qy, 0.0, hc, ok);
         sUC[idx] = f.u;
         sUC[PS + idx] = f.v;
@@ -769,7 +770,7 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
         }
         {  // friction and erosion/deposition from U^n
             double k1 = vk[1], k2 = vk[2], phi;
-            if (P.manning || !wet_divisor(v0[0]) || !sources<true>(P, dt, v0, k1, k2, phi)) {
+            if (P.manning || !sources<true>(P, dt, v0, k1, k2, phi)) {
                 State5 v;
                 v.h = v0[0];
                 v.qx = v0[1];
@@ -823,12 +824,10 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
         }
         double d;  // last stage: the new cell's CFL step
         {
-            bool ok = wet_divisor(h);
-            double fh = h, fx = qx, fy = qy, fc = hc;
-            if (ok) {
-                const Face5 f = filter_face<true>(fh, fx, fy, z, fc, ok);
-                if (LAST) ok &= cfl_dt_fast(P, f, d);
-            }
+            bool ok = true;
+            double fh = (h < 0.0) ? 0.0 : h, fx = qx, fy = qy, fc = hc;
+            const Face5 f = filter_face<true>(fh, fx, fy, z, fc, ok);
+            if (LAST) ok &= cfl_dt_fast(P, f, d);
             if (!ok) {
                 fh = h;
                 fx = qx;
