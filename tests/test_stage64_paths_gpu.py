@@ -83,3 +83,27 @@ def test_periodic_seam_with_an_expired_series(rk):
     o.run(3)
     for f in range(5):
         assert np.array_equal(V[f], o.V[f]), (f, np.abs(V[f] - o.V[f]).max())
+
+
+@pytest.mark.parametrize("nx,ny", [(37, 13), (545, 171)])
+@pytest.mark.parametrize("order", [2, 1])
+def test_grass_law_at_fronts_equals_the_oracle(nx, ny, order):
+    """Grass's bed flux has no depth in it: water that moves below the bed of
+    the dry cell beside it moves sediment, where every other flux is a zero."""
+    w = mixed_state(nx, ny, nx + 7)
+    w.mask = np.ones((ny, nx), dtype=np.int32)
+    sw = make_switches(order=order, wbc=1, read_files=0, bedload_law=1, grass_ag=1e-3)
+    s = T.Solver(w.p, sw)
+    try:
+        s.set_state(w.V)
+        s.set_mask(w.mask)
+        s.reset()
+        k = s.consts()
+        s.step(4)
+        V = s.state()
+    finally:
+        s.close()
+    o = oracle.OracleRun(w.p, sw, w.V, w.mask, None, None, kconsts=k)
+    o.run(4)
+    for f in range(5):
+        assert np.array_equal(V[f], o.V[f]), (f, np.abs(V[f] - o.V[f]).max())

@@ -309,10 +309,12 @@ __device__ __forceinline__ bool edge_flux(const Phys64 &P, const Face5 &a, const
     h0 = (h0 > 0.0) ? h0 : 0.0;  // fmax(h0, 0)
     h1 = (h1 > 0.0) ? h1 : 0.0;
     const double deta = h1 - h0;
-    if (FAST && h0 == 0.0 && h1 == 0.0) {
+    if (FAST && h0 == 0.0 && h1 == 0.0 && (P.bedload_law == 0 || (a.u == 0.0 && b.u == 0.0))) {
         // no water stands against either side (both faces dry, or water below
         // the other side's bed): F and DU are zeros, and so is everything the
-        // finite wave speeds multiply.  Dry land makes this a common edge.
+        // finite wave speeds multiply (the Grass law's bed flux has no depth in
+        // it: there the water has to stand still too).  Dry land makes this a
+        // common edge.
         const double z = 0.0 * (a.u + a.v + a.c + b.u + b.v + b.c);
 #pragma unroll
         for (int i = 0; i < 5; i++) Dm[i] = Dp[i] = z;
