@@ -48,6 +48,7 @@ namespace tsu {
 template <int TX_, int TY_, int NTHR_ = TX_ * TY_>
 struct Tile {
     static constexpr int TX = TX_, TY = TY_, NT = NTHR_;
+    static constexpr bool kSmall = TX * TY <= 64;  // the small grids' tile
     static_assert(NTHR_ >= TX_ * TY_ && NTHR_ % 32 == 0 && NTHR_ <= 1024, "threads per tile");
     static constexpr int LX = TX + 4, LY = TY + 4, PS = LX * LY;  // loaded tile, 2-cell halo
     static constexpr int FXW = TX + 2, FYH = TY + 2;               // faces incl. one halo cell
@@ -156,8 +157,9 @@ __device__ __forceinline__ Face5 to_y(const Face5 &f) {
     r.v = -f.u;
     return r;
 }
-template <bool FAST>
+template <bool FAST, bool FRONT = false>
 __device__ __forceinline__ Face5 filtered(State5 &s, bool &ok) {
+    if (FRONT) return filter_near_front(s.h, s.qx, s.qy, s.H, s.hc, ok);
     return filter_face<FAST>(s.h, s.qx, s.qy, s.H, s.hc, ok);
 }
 
@@ -166,7 +168,7 @@ __device__ __forceinline__ Face5 filtered(State5 &s, bool &ok) {
 // valid.  qplus / qminus (may be null): the discharges of the plus-side face
 // normal to its edge and of the minus-side face along it, for the periodic
 // seam (ydir: the direction is y).
-template <int PS, bool FAST>
+template <int PS, bool FAST, bool FRONT = false>
 __device__ __forceinline__ bool make_faces(const double *sV, const double *sUC, int c, int step, double *dst,
                                            int fstride, int side, double *deta_out, double *qplus = nullptr,
                                            double *qminus = nullptr) {
@@ -174,7 +176,7 @@ __device__ __forceinline__ bool make_faces(const double *sV, const double *sUC, 
     State5 m, p;
     double deta;
     reconstruct_dir<PS, FAST>(sV, sUC, c, c - step, c + step, m, p, deta, ok);
-    Face5 fm = filtered<FAST>(m, ok), fp = filtered<FAST>(p, ok);  // GPU/Reconstructor.cu:344-348
+    Face5 fm = filtered<FAST, FRONT>(m, ok), fp = filtered<FAST, FRONT>(p, ok);  // GPU/Reconstructor.cu:344-348
     if (step != 1) {
         fm = to_y(fm);
         fp = to_y(fp);
@@ -186,9 +188,14 @@ __device__ __forceinline__ bool make_faces(const double *sV, const double *sUC, 
     if (qminus) *qminus = (step != 1) ? m.qx : m.qy;
     return ok;
 }
-template <int PS>
+// FRONT: the near_front form first.  It pays on the small grids' tile, where one
+// face by the ordinary operators sets the time of the stage (48 x 36 cells with
+// a coast: 23.0 -> 19.7 us per step); the large tile's warps hide it, and its
+// registers cost them 2 %.
+template <int PS, bool FRONT>
 __device__ __noinline__ void make_faces_any(const double *sV, const double *sUC, int c, int step, double *dst,
                                             int fstride, int side, double *deta_out, double *qplus, double *qminus) {
+    if (FRONT && make_faces<PS, true, true>(sV, sUC, c, step, dst, fstride, side, deta_out, qplus, qminus)) return;
     make_faces<PS, false>(sV, sUC, c, step, dst, fstride, side, deta_out, qplus, qminus);
 }
 
@@ -214,19 +221,26 @@ __device__ __noinline__ void put_edge_any(const Phys64 &P, Face5 a, Face5 b, int
 // Friction (GPU/Reconstructor.cu:33-55) on the momentum (k1, k2) and the
 // erosion/deposition rate phi (:57-88), from U^n = v0; one velocity
 // evaluation serves both.
-template <bool FAST>
+template <bool FAST, bool FRONT = false>
 __device__ __forceinline__ bool sources(const Phys64 &P, double dt, const double v0[5], double &k1, double &k2,
                                         double &phi) {
     bool ok = true;
     double ux, uy, modu;
     const Divisor<FAST> d0(v0[0] + kEpsilon, ok);
-    if (FAST) {
-        ux = d0.of(v0[1]);
-        uy = d0.of(v0[2]);
+    if constexpr (FAST) {
+        if constexpr (FRONT) {
+            Divisor<true> dv = d0;
+            velocity_near_front(v0[0], v0[1], v0[2], dv, ux, uy, ok);
+        } else {
+            ux = d0.of(v0[1]);
+            uy = d0.of(v0[2]);
+        }
         const double m2 = ux * ux + uy * uy;
         // an empty cell: every quotient by EPSILON or eps_h is a zero
-        ok &= (wet_divisor(d0.d) & calm(v0[1], ux) & calm(v0[2], uy) & mid_or_zero(m2)) |
-              (empty(v0[0], v0[1], v0[2], v0[4]) & mid(P.eps_h));
+        if constexpr (FRONT) ok &= mid_or_zero(m2) & mid(v0[0] + P.eps_h);
+        else
+            ok &= (wet_divisor(d0.d) & calm(v0[1], ux) & calm(v0[2], uy) & mid_or_zero(m2)) |
+                  (empty(v0[0], v0[1], v0[2], v0[4]) & mid(P.eps_h));
         modu = root(m2);
     } else {
         velocity(v0[0], v0[1], v0[2], ux, uy);
@@ -266,9 +280,13 @@ __device__ __forceinline__ bool sources(const Phys64 &P, double dt, const double
 struct Sources {
     double k1, k2, phi;
 };
+template <bool FRONT>
 __device__ __noinline__ Sources sources_any(const Phys64 &P, double dt, State5 v, double k1, double k2) {
     const double v0[5] = {v.h, v.qx, v.qy, v.H, v.hc};
     Sources r;
+    r.k1 = k1;
+    r.k2 = k2;
+    if (FRONT && !P.manning && sources<true, true>(P, dt, v0, r.k1, r.k2, r.phi)) return r;
     r.k1 = k1;
     r.k2 = k2;
     sources<false>(P, dt, v0, r.k1, r.k2, r.phi);
@@ -559,7 +577,7 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
             } else {
                 double *deta = (didx >= 0) ? sDeta + didx : nullptr;
                 if (seam_q || !make_faces<PS, true>(sV, sUC, c, step, dst, fstride, side, deta))
-                    make_faces_any<PS>(sV, sUC, c, step, dst, fstride, side, deta, qplus, qminus);
+                    make_faces_any<PS, T::kSmall>(sV, sUC, c, step, dst, fstride, side, deta, qplus, qminus);
             }
         } else {  // first order: faces are the cell values (GPU/Reconstructor.cu:99-107)
             Face5 f;
@@ -777,7 +795,7 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
                 v.qy = v0[2];
                 v.H = v0[3];
                 v.hc = v0[4];
-                const Sources r = sources_any(P, dt, v, vk[1], vk[2]);
+                const Sources r = sources_any<T::kSmall>(P, dt, v, vk[1], vk[2]);
                 k1 = r.k1;
                 k2 = r.k2;
                 phi = r.phi;
