@@ -576,7 +576,6 @@ __global__ void __launch_bounds__(kWgThreads, 1)
     const TileGeom G = tile_geom(nimg, H, W);
     const int ntile = (int)blockIdx.x < G.total ? (G.total - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
 
-    if (warp == 1) tmem_alloc(tslot, 256);
     if (tid == 0) {
         for (int k = 0; k < 2; k++) {
             mbar_init(&accf[k], 1);
@@ -591,10 +590,15 @@ __global__ void __launch_bounds__(kWgThreads, 1)
         *sFail = 0;
         mbar_init_fence();
     }
+    // TMEM is taken only now: a grid that holds some while it waits could starve
+    // the one it waits for, if that one lets it start before it has its own
+    prior_grids_done();
+    if (warp == 1) tmem_alloc(tslot, 256);
     fence_before();
     __syncthreads();
     fence_after();
     const uint32_t tmem = *tslot;
+    next_grid_may_start();
     float db[32];      // bias gradient of this thread's pixels
     float sum[3][32];  // this lane's row of D (j, cout), summed over the batches
 #pragma unroll
@@ -1061,6 +1065,8 @@ __global__ void __launch_bounds__(32 * kRedWarps)
     const bool bias = k >= 32 * KROWS;  // the last block
     const int n = bias ? 4 * nctas : nctas;
     float acc = 0.f;
+    prior_grids_done();
+    next_grid_may_start();
     for (int b0 = w; b0 < n; b0 += kRedWarps * kRedRows) {
         float v[kRedRows];
 #pragma unroll
@@ -1144,10 +1150,13 @@ cudaError_t wgrad_launch(const bf16 *X, const bf16 *dZ, int nimg, int H, int W, 
         if (e != cudaSuccess) return e;
         part = own;
     }
-    conv3x3_wgrad_kernel<<<ctas, kWgThreads, kWgSmem, st>>>(mx, mz, nimg, H, W, part);
+    // programmatic dependent launches: the reduction's blocks are in place when
+    // the partials are complete (8 images of 528^2: 76.2 -> 73.5 us; the same for
+    // the forward kernel cost it 1 %)
+    launch_after(conv3x3_wgrad_kernel, dim3(ctas), dim3(kWgThreads), kWgSmem, st, mx, mz, nimg, H, W, part);
     e = cudaGetLastError();
     if (e == cudaSuccess) {
-        wgrad_reduce_kernel<<<KROWS + 1, 32 * kRedWarps, 0, st>>>(part, ctas, dW, db, add);
+        launch_after(wgrad_reduce_kernel, dim3(KROWS + 1), dim3(32 * kRedWarps), 0, st, part, ctas, dW, db, add);
         e = cudaGetLastError();
     }
     if (own) {
