@@ -20,14 +20,14 @@
 // whose M = 128 rows are 16 groups of 8 pixels of one image row each and whose
 // N = 96 columns are the contributions of an input row to the three output
 // rows around it, 6 MMAs (3 column offsets x 2 channel halves, K = 16) per
-// input row.  8 x 528^2 pixels, BF16 with ReLU: 105 -> 69 us from HBM (the 285
-// MB it reads and writes take 44 us), 98 -> 57 us when the input is in L2.
+// input row.  8 x 528^2 pixels, BF16 with ReLU: 103 -> 65 us from HBM (the 285
+// MB it reads and writes take 44 us).
 //
 // Weight gradient (conv3x3_wgrad_kernel): dW[cout][tap][cin] =
 //   sum_p dZ[p][cout] X[p + off(tap)][cin], a GEMM with the pixels as the
 // reduction dimension; all nine taps in one MMA per 16 pixels (M = the three
 // row offsets x cin, N = the three column offsets x cout).  8 x 528^2: kernel
-// 100 -> 50 us, the call with its reduction 185 -> 75 us.  The bias gradient
+// 100 -> 50 us, the call with its reduction 187 -> 74 us.  The bias gradient
 // is summed from the dZ tile on the CUDA cores.
 //
 // Every mbarrier wait is bounded (globaltimer); on expiry the kernel sets
@@ -89,9 +89,11 @@ constexpr int kWgStages = 8;
 constexpr int kWgThreads = 192;
 // tiles summed in TMEM before the sum moves to registers: the tensor cores add
 // to an FP32 accumulator with truncation, whose bias grows with the number of
-// additions (8 x 528^2: relative error of dW against 64 bits 1.4e-5 with all
-// 118 tiles of a CTA in one accumulator, 3e-6 with at most 30)
-constexpr int kWgFlush = 24;
+// additions.  Relative error of dW against 64 bits at 8 x 528^2 / 1 x 428 x 330:
+// all of a CTA's tiles in one accumulator 1.4e-5, batches of 24 2.3e-6 /
+// 6.3e-7, of 8 6.5e-7 / 6.3e-7, of 6 4.9e-7 / 4.3e-7 (592 CTAs with an
+// accumulator each 3.2e-6 / 4.8e-7); 62-63 us warm for any of them
+constexpr int kWgFlush = 6;
 constexpr int kWgSmem = 1024 + kWgStages * kWgStage + (2 * kWgStages + 5) * 8 + 32;
 static_assert(kXBuf % 512 == 0 && kWgStage % 512 == 0, "swizzled TMA destinations");
 static_assert(kWgSmem + 1024 <= 228 * 1024, "one CTA per SM");

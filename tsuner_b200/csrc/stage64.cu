@@ -28,9 +28,9 @@
 // roots per cell and stage.  They are evaluated without branches and with
 // shared reciprocals (ieee64.h), each phase with one test that sends the
 // operands it cannot take to a general form of the same formulas.  4096^2,
-// the N-wave entering still water, 2 steps: 12.1 -> 9.6 ms; 1021 x 773 with
-// currents everywhere, 4 steps: 1350 -> 943 us (FP64 pipe 34 -> 46 % busy, 117
-// -> 87 warp instructions per cell in the first stage).
+// the N-wave entering still water, 2 steps: 12.1 -> 8.9 ms; 1021 x 773 with
+// currents everywhere, 4 steps: 1356 -> 900 us (FP64 pipe 34 -> 50 % busy, 117
+// -> 88 warp instructions per cell in the first stage, 60 % issue).
 #include <cuda_runtime.h>
 
 #include <cstdlib>
