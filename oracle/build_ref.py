@@ -150,8 +150,8 @@ def main(argv=None):
     ap.add_argument("--force", action="store_true")
     ap.add_argument("variants", nargs="*", help="kernel variants (and/or 'interp'); default: all")
     a = ap.parse_args(argv)
-    if not os.path.isdir(a.ref):
-        print("reference tree not present; keeping prebuilt oracle/_ref")
+    if not os.path.isdir(os.path.join(a.ref, "GPU")):
+        print("reference sources not present; keeping prebuilt oracle/_ref")
         return 0
     names = a.variants or [v + sfx for v in VARIANTS for sfx in ("", "-nolto")] + ["interp"]
     for v in names:
