@@ -152,8 +152,26 @@ __device__ __forceinline__ void tma_load_5d(void *dst, const CUtensorMap *map, i
 // writes are visible; nothing it wrote, and nothing it may still read, is
 // touched before.  next_grid_may_start() lets the kernel after this one take
 // the SM slots that this one's CTAs leave.
+// What an earlier kernel of the chain writes is not read-only for the whole
+// life of this one, so it is not read through __ldg or a const __restrict__
+// pointer (ld.global.nc: neither the compiler nor the SM's read-only path has
+// to keep such a load behind the wait), nor through __ldcg (not ordered by the
+// compiler): ordinary loads, TMA, or load_written() below.  __ldg is for what
+// only the host writes: mask, series, descriptors.
 __device__ __forceinline__ void prior_grids_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void next_grid_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// A coherent load from L2, kept in program order behind prior_grids_done().
+__device__ __forceinline__ float load_written(const float *p) {
+    float v;
+    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double load_written(const double *p) {
+    double v;
+    asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
 
 template <typename... P, typename... A>
 cudaError_t launch_after(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {

@@ -1059,8 +1059,7 @@ cudaError_t conv_launch(ConvArgs a, cudaStream_t st) {
 // latency, not a bandwidth), then the sums are added in order.
 constexpr int kRedWarps = 16, kRedRows = 10;  // one pass covers 160 rows
 __global__ void __launch_bounds__(32 * kRedWarps)
-    wgrad_reduce_kernel(const float *__restrict__ part, int nctas, float *__restrict__ dW, float *__restrict__ db,
-                        bool add) {
+    wgrad_reduce_kernel(const float *part, int nctas, float *dW, float *db, bool add) {
     __shared__ float sSum[kRedWarps][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int k = blockIdx.x * 32 + lane;
@@ -1076,7 +1075,7 @@ __global__ void __launch_bounds__(32 * kRedWarps)
             const int b = b0 + i * kRedWarps;
             const float *p = bias ? part + (size_t)(b >> 2) * kWgPart + 32 * KROWS + (b & 3) * 32 + lane
                                   : part + (size_t)b * kWgPart + k;
-            v[i] = (b < n) ? __ldcg(p) : 0.f;
+            v[i] = (b < n) ? tsu::load_written(p) : 0.f;
         }
 #pragma unroll
         for (int i = 0; i < kRedRows; i++) acc += v[i];

@@ -181,7 +181,7 @@ __device__ __forceinline__ void stage32_tile(const Stage32Args &A, const Phys32 
         V0 = A.bufA;
         Vout = FIRST ? A.bufB : A.bufA;
     } else {
-        par = (int)__ldcg(A.scal + SC_PAR);
+        par = (int)load_written(A.scal + SC_PAR);
         Vin = par ? A.bufB : A.bufA;
         V0 = Vin;
         Vout = par ? A.bufA : A.bufB;
@@ -215,7 +215,7 @@ __device__ __forceinline__ void stage32_tile(const Stage32Args &A, const Phys32 
             }
             const long long g = (long long)gy * pitch + gx;
 #pragma unroll
-            for (int f = 0; f < 5; f++) sV[f * PS + idx] = __ldg(Vin + f * plane + g);
+            for (int f = 0; f < 5; f++) sV[f * PS + idx] = load_written(Vin + f * plane + g);
             sM[ly * MLX + lxc + (MHX - 2)] = __ldg(A.mask + g);
         }
     }
@@ -236,7 +236,8 @@ __device__ __forceinline__ void stage32_tile(const Stage32Args &A, const Phys32 
         prefetch_l2(A.eta_max + gown);
     }
     // the scalars are read while the box travels
-    const double t = __ldcg(A.scal + SC_T), tend = __ldcg(A.scal + SC_TEND), dtd = __ldcg(A.scal + SC_DT);
+    const double t = load_written(A.scal + SC_T), tend = load_written(A.scal + SC_TEND);
+    const double dtd = load_written(A.scal + SC_DT);
     const float dt = (float)dtd;
     __syncthreads();
     if (use_tma) {  // every thread sees the box land (bounded wait)
@@ -511,12 +512,12 @@ __device__ __forceinline__ void stage32_tile(const Stage32Args &A, const Phys32 
     if (own) {
         float v0[5];
 #pragma unroll
-        for (int f = 0; f < 5; f++) v0[f] = FIRST ? vc[f] : __ldcg(V0 + f * plane + gown);
+        for (int f = 0; f < 5; f++) v0[f] = FIRST ? vc[f] : load_written(V0 + f * plane + gown);
         float ex_h = 0.f, ex_b = 0.f, ex_e = 0.f;
         if (LAST) {
-            ex_h = __ldcg(A.hmax + gown);
-            ex_b = __ldcg(A.bmin + gown);
-            ex_e = __ldcg(A.eta_max + gown);
+            ex_h = load_written(A.hmax + gown);
+            ex_b = load_written(A.bmin + gown);
+            ex_e = load_written(A.eta_max + gown);
         }
         float z = vc[0], H = vc[1], qx = vc[2], qy = vc[3], hc = vc[4];
         if (ORDER == 2) {
