@@ -44,8 +44,9 @@ struct TsuEnsemble {
     int *d_tile_member = nullptr;
     unsigned *d_work = nullptr;
     unsigned ntiles = 0;
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t graph_exec = nullptr;
+    // captured steps: [0] without, [1] with an end time (EnsArgs::until)
+    cudaGraph_t graph[2] = {};
+    cudaGraphExec_t graph_exec[2] = {};
     long last_launches = 0;
     bool timed = false;
     int num_sms = 148;
@@ -87,10 +88,12 @@ void ens_error(const char *fmt, ...) {
     } while (0)
 
 void drop_graph(TsuEnsemble *E) {
-    if (E->graph_exec) cudaGraphExecDestroy(E->graph_exec);
-    if (E->graph) cudaGraphDestroy(E->graph);
-    E->graph_exec = nullptr;
-    E->graph = nullptr;
+    for (int q = 0; q < 2; q++) {
+        if (E->graph_exec[q]) cudaGraphExecDestroy(E->graph_exec[q]);
+        if (E->graph[q]) cudaGraphDestroy(E->graph[q]);
+        E->graph_exec[q] = nullptr;
+        E->graph[q] = nullptr;
+    }
 }
 
 // Rebuilds the member descriptors and the global tile list for `variant`.
@@ -166,7 +169,7 @@ int refresh_members(TsuEnsemble *E) {
     return TSU_OK;
 }
 
-EnsArgs ens_args(const TsuEnsemble *E) {
+EnsArgs ens_args(const TsuEnsemble *E, bool until) {
     EnsArgs a;
     a.members = E->d_members;
     a.tile_member = E->d_tile_member;
@@ -174,11 +177,12 @@ EnsArgs ens_args(const TsuEnsemble *E) {
     a.dynamic = E->dynamic;
     a.work = E->d_work;
     a.tmas = E->d_tmas;
+    a.until = until;
     return a;
 }
 
-int launch_steps(TsuEnsemble *E, long nsteps) {
-    const EnsArgs a = ens_args(E);
+int launch_steps(TsuEnsemble *E, long nsteps, bool until = false) {
+    const EnsArgs a = ens_args(E, until);
     const int order = E->m[0]->sw.order;
     for (long i = 0; i < nsteps; i++)
         for (int k = 0; k < order; k++) ECK(ens32_launch(E->variant, order, k, a, E->m[0]->phys32, E->ctas, E->st));
@@ -310,8 +314,7 @@ extern "C" int tsu_ens_get_config(TsuEnsemble *E, int *variant, int *tx, int *ty
     return TSU_OK;
 }
 
-extern "C" int tsu_ens_step(TsuEnsemble *E, long nsteps) {
-    if (!E || nsteps < 0) return TSU_ERR_INVALID;
+static int ens_step(TsuEnsemble *E, long nsteps, bool until) {
     for (TsuSolver *s : E->m)
         if (!s->ready) return TSU_ERR_INVALID;  // tsu_ens_reset first
     ECK(cudaSetDevice(E->device));
@@ -319,27 +322,32 @@ extern "C" int tsu_ens_step(TsuEnsemble *E, long nsteps) {
     if (rc0) return rc0;
     const long K = TsuSolver::kGraphSteps;
     long n = nsteps;
-    if (n >= K && !E->graph_exec) {  // host-side setup, once: before the timed region
+    if (n >= K && !E->graph_exec[until]) {  // host-side setup, once: before the timed region
         ECK(cudaStreamBeginCapture(E->st, cudaStreamCaptureModeThreadLocal));
-        int rc = launch_steps(E, K);
+        int rc = launch_steps(E, K, until);
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamEndCapture(E->st, &g);
         if (rc) return rc;
         ECK(e);
-        E->graph = g;
-        ECK(cudaGraphInstantiate(&E->graph_exec, g, 0));
+        E->graph[until] = g;
+        ECK(cudaGraphInstantiate(&E->graph_exec[until], g, 0));
     }
     ECK(cudaEventRecord(E->e0, E->st));
-    while (n >= K && E->graph_exec) {
-        ECK(cudaGraphLaunch(E->graph_exec, E->st));
+    while (n >= K && E->graph_exec[until]) {
+        ECK(cudaGraphLaunch(E->graph_exec[until], E->st));
         n -= K;
     }
-    int rc = launch_steps(E, n);
+    int rc = launch_steps(E, n, until);
     if (rc) return rc;
     ECK(cudaEventRecord(E->e1, E->st));
     E->last_launches = nsteps * E->m[0]->sw.order * (E->dynamic ? 2 : 1);
     E->timed = true;
     return TSU_OK;
+}
+
+extern "C" int tsu_ens_step(TsuEnsemble *E, long nsteps) {
+    if (!E || nsteps < 0) return TSU_ERR_INVALID;
+    return ens_step(E, nsteps, false);
 }
 
 extern "C" int tsu_ens_sync(TsuEnsemble *E) {
@@ -503,7 +511,7 @@ extern "C" int tsu_ens_run_until(TsuEnsemble *E, double t_end, long max_steps, l
     long done_steps = 0;
     while (e == cudaSuccess && !rc && done_steps < max_steps) {
         const long chunk = std::min<long>(64, max_steps - done_steps);
-        rc = tsu_ens_step(E, chunk);
+        rc = ens_step(E, chunk, true);
         if (rc) break;
         done_steps += chunk;
         all_done_kernel<<<1, 256, 0, E->st>>>(E->d_members, E->n, t_end, d_done);

@@ -804,7 +804,13 @@ extern "C" int tsu_run_until(TsuSolver *s, double t_end, long max_steps, long *s
     long left = max_steps;
     int rf = TSU_OK;
     while (left > 0) {
+        // No more steps than the current dt needs to reach t_end (and one): a
+        // step past it changes nothing but loads every tile before it can know
+        // (4096^2 FP64: 0.6 ms each of up to 63).  Falling short costs one more
+        // round of this loop.
         long chunk = left < 64 ? left : 64;
+        const double need = (t_end - sc[SC_T]) / sc[SC_DT];
+        if (need < (double)(chunk - 1)) chunk = need > 0.0 ? (long)need + 2 : 1;
         int r = tsu_step(s, chunk);
         if (r) return r;
         left -= chunk;
