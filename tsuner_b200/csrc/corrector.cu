@@ -1017,23 +1017,44 @@ cudaError_t make_map(CUtensorMap *m, const void *base, int nimg, int H, int W, i
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+// What is set up or looked up once per device: the kernels' shared-memory
+// attribute, the SM count, the pool of the calls that bring no scratch.
+constexpr int kMaxDevices = 64;
+struct DeviceState {
+    bool ready = false;
+    int sms = 0;
+    cudaMemPool_t pool = nullptr;
+};
+std::mutex g_dev_mu;
+DeviceState g_dev[kMaxDevices];
+// the current device's entry, or null (a device beyond the table: looked up on each call)
+DeviceState *device_state() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
+    return &g_dev[dev];
+}
+
+// the kernels' shared memory on the current device
 cudaError_t prepare() {
-    static bool done = false;
-    if (done) return cudaSuccess;
+    std::lock_guard<std::mutex> g(g_dev_mu);
+    DeviceState *d = device_state();
+    if (d && d->ready) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(conv3x3_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(conv3x3_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem);
-    if (e == cudaSuccess) done = true;
+    if (e == cudaSuccess && d) d->ready = true;
     return e;
 }
 
+// SMs of the current device
 int num_sms() {
-    static int n = 0;
-    if (!n) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 148;
-    }
+    std::lock_guard<std::mutex> g(g_dev_mu);
+    DeviceState *d = device_state();
+    if (d && d->sms) return d->sms;
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 148;
+    if (d) d->sms = n;
     return n;
 }
 
@@ -1098,39 +1119,35 @@ int wgrad_ctas(int nimg, int H, int W) { return std::min(tile_geom(nimg, H, W).t
 // maps it again (600 us against 80 us for the gradient itself); this pool
 // keeps up to kKeep bytes (one unit of its growth).  tsu_corr_destroy returns them.
 constexpr unsigned long long kKeep = 32ull << 20;
-constexpr int kMaxDevices = 64;
-std::mutex g_pool_mu;
-cudaMemPool_t g_pool[kMaxDevices] = {};
 
 cudaError_t scratch_alloc(float **p, size_t bytes, cudaStream_t st) {
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (st && cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
     cudaMemPool_t pool = nullptr;
-    if (cap == cudaStreamCaptureStatusNone && dev < kMaxDevices) {
-        std::lock_guard<std::mutex> g(g_pool_mu);
-        if (!g_pool[dev]) {
+    std::unique_lock<std::mutex> g(g_dev_mu);
+    DeviceState *d = device_state();
+    if (cap == cudaStreamCaptureStatusNone && d) {
+        if (!d->pool) {
             cudaMemPoolProps props{};
             props.allocType = cudaMemAllocationTypePinned;
             props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = dev;
+            props.location.id = (int)(d - g_dev);
             unsigned long long keep = kKeep;
-            if (cudaMemPoolCreate(&g_pool[dev], &props) != cudaSuccess) {
+            if (cudaMemPoolCreate(&d->pool, &props) != cudaSuccess) {
                 cudaGetLastError();
-                g_pool[dev] = nullptr;
+                d->pool = nullptr;
             } else {
-                cudaMemPoolSetAttribute(g_pool[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+                cudaMemPoolSetAttribute(d->pool, cudaMemPoolAttrReleaseThreshold, &keep);
             }
         }
-        pool = g_pool[dev];
+        pool = d->pool;
     }
+    g.unlock();
     return pool ? cudaMallocFromPoolAsync((void **)p, bytes, pool, st) : cudaMallocAsync((void **)p, bytes, st);
 }
 void scratch_trim(int dev) {
-    std::lock_guard<std::mutex> g(g_pool_mu);
-    if (dev >= 0 && dev < kMaxDevices && g_pool[dev]) cudaMemPoolTrimTo(g_pool[dev], 0);
+    std::lock_guard<std::mutex> g(g_dev_mu);
+    if (dev >= 0 && dev < kMaxDevices && g_dev[dev].pool) cudaMemPoolTrimTo(g_dev[dev].pool, 0);
 }
 
 // part: wgrad_ctas(...) * kWgPart floats of device scratch, or null (then
