@@ -56,9 +56,36 @@ static int threads() {
     return 0;
 }
 
+// a prediction's device memory: one map (16 B per fine cell) for one sample,
+// two for several, one again where there is no room for two
+static int predict_memory() {
+    const int n = 64;
+    const size_t np = (size_t)n * n, map = 16 * np;
+    std::vector<float> H(np, 1.f), coarse(3 * 3 * np / 16, 1.f), out(6 * np);
+    for (int room = 1; room <= 2; room++) {
+        TsuCorrector *c = nullptr;
+        EXPECT(tsu_corr_create(&c, n, n, 4, 1, 7, 0) == TSU_OK);
+        EXPECT(tsu_corr_set_site(c, H.data()) == TSU_OK);
+        EXPECT(tsu_corr_add_samples(c, 3, coarse.data(), nullptr) == TSU_OK);
+        const size_t before = fake::in_use;
+        fake::memory = before + room * map;
+        EXPECT(tsu_corr_predict(c, 0, 1, out.data(), out.data() + 3 * np, nullptr, nullptr) == TSU_OK);
+        EXPECT(fake::in_use == before + map);
+        fake::launches.clear();
+        EXPECT(tsu_corr_predict(c, 0, 3, out.data(), out.data() + 3 * np, nullptr, nullptr) == TSU_OK);
+        EXPECT(fake::in_use == before + room * map);
+        EXPECT(fake::launches.size() == 3 * 8);  // features, six layers, the map
+        EXPECT(tsu_corr_destroy(c) == TSU_OK);
+        EXPECT(fake::blocks.empty());
+        fake::memory = ~(size_t)0;
+    }
+    return 0;
+}
+
 int main(int argc, char **argv) {
     const char *s = argc > 1 ? argv[1] : "";
     if (!std::strcmp(s, "two_devices")) return two_devices();
     if (!std::strcmp(s, "threads")) return threads();
+    if (!std::strcmp(s, "predict_memory")) return predict_memory();
     return 2;
 }

@@ -30,3 +30,7 @@ def check(tmp_path_factory):
 @pytest.mark.parametrize("scenario", ["two_devices", "threads"])
 def test_every_device_is_set_up(check, scenario):
     check(scenario)
+
+
+def test_a_prediction_takes_the_memory_it_needs(check):
+    check("predict_memory")

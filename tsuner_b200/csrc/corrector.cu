@@ -1229,8 +1229,9 @@ struct TsuCorrector {
     float *E = nullptr;
     int env_n = 0, ntrain = 0;
     float *wg_part = nullptr;  // weight-gradient partials of one layer ([CTAs][kWgPart])
-    // predictions: two maps of one sample each ([4][H*W]), so that one is copied
-    // to the host (on cp) while the next is computed; made at the first prediction
+    // predictions: a map of one sample ([4][H*W]), made at the first prediction,
+    // and a second one at the first of several samples, so that one is copied
+    // to the host (on cp) while the next is computed
     float *out[2] = {};
     cudaStream_t cp = nullptr;
     cudaEvent_t done[2] = {};
@@ -1596,28 +1597,34 @@ extern "C" int tsu_corr_predict(TsuCorrector *c, int first, int n, float *out_hm
         const int r = compute_envelope(c, c->ntrain);
         if (r) return r;
     }
-    if (!c->cp) {
-        for (int q = 0; q < 2; q++) {
-            if (!c->out[q]) CCK(cudaMalloc((void **)&c->out[q], 4 * np * 4));
+    if (!c->out[0]) CCK(cudaMalloc((void **)&c->out[0], 4 * np * 4));
+    if (n > 1 && !c->out[1] && cudaMalloc((void **)&c->out[1], 4 * np * 4) != cudaSuccess) {
+        cudaGetLastError();  // no room for it: one sample after the other
+        c->out[1] = nullptr;
+    }
+    const bool two = n > 1 && c->out[1];
+    if (two && !c->cp) {
+        for (int q = 0; q < 2; q++)
             if (!c->done[q]) CCK(cudaEventCreateWithFlags(&c->done[q], cudaEventDisableTiming));
-        }
         CCK(cudaStreamCreateWithFlags(&c->cp, cudaStreamNonBlocking));
     }
-    auto compute = [&](int k) -> int {  // sample first + k -> out[k & 1]
+    const cudaStream_t copy = two ? c->cp : c->st;
+    auto map = [&](int k) { return two ? k & 1 : 0; };
+    auto compute = [&](int k) -> int {  // sample first + k -> its map
         const int s = first + k;
         int r = load_batch(c, &s, 1, false);
         if (!r) r = forward(c, 1);
         if (r) return r;
         apply_kernel<<<2 * num_sms(), 256, 0, c->st>>>(c->Yout, c->base, c->cv, c->clip_depth, clamp ? c->E : nullptr,
-                                                         c->envelope, c->out[k & 1]);
+                                                         c->envelope, c->out[map(k)]);
         CCK(cudaGetLastError());
-        CCK(cudaEventRecord(c->done[k & 1], c->st));
+        if (two) CCK(cudaEventRecord(c->done[map(k)], c->st));
         return TSU_OK;
     };
     int rc = compute(0);
     for (int k = 0; k < n && !rc; k++) {
         // the other map's copy (of sample k - 1) has ended: planes_d2h waits for it
-        if (k + 1 < n) rc = compute(k + 1);
+        if (two && k + 1 < n) rc = compute(k + 1);
         if (rc) break;
         float *want[4] = {out_hmax, out_db, base_hmax, base_db};
         void *outs[4];
@@ -1626,15 +1633,16 @@ extern "C" int tsu_corr_predict(TsuCorrector *c, int first, int n, float *out_hm
         for (int q = 0; q < 4; q++)
             if (want[q]) {
                 outs[m] = want[q] + k * np;
-                ins[m++] = c->out[k & 1] + q * np;
+                ins[m++] = c->out[map(k)] + q * np;
             }
-        if (cudaStreamWaitEvent(c->cp, c->done[k & 1], 0) != cudaSuccess ||
-            tsu::planes_d2h(m, outs, (size_t)c->W * 4, ins, (size_t)c->W * 4, (size_t)c->W * 4, c->H, c->cp) != cudaSuccess ||
-            cudaStreamSynchronize(c->cp) != cudaSuccess) {
+        if ((two && cudaStreamWaitEvent(copy, c->done[map(k)], 0) != cudaSuccess) ||
+            tsu::planes_d2h(m, outs, (size_t)c->W * 4, ins, (size_t)c->W * 4, (size_t)c->W * 4, c->H, copy) != cudaSuccess ||
+            cudaStreamSynchronize(copy) != cudaSuccess) {
             snprintf(g_corr_msg, sizeof(g_corr_msg), "tsu_corr_predict: CUDA error");
             rc = TSU_ERR_CUDA;
             break;
         }
+        if (!two && k + 1 < n) rc = compute(k + 1);
     }
     if (cudaStreamSynchronize(c->st) != cudaSuccess && !rc) {
         snprintf(g_corr_msg, sizeof(g_corr_msg), "tsu_corr_predict: CUDA error");
