@@ -79,6 +79,11 @@ TSU_HD bool mid_or_zero(double x) {
     const uint32_t t = hi32(x) & 0x7fffffffu;
     return (t - 0x0df00000u < 0x64000000u) | ((t | lo32(x)) == 0u);
 }
+// 2^-800 <= |x| < 2^80, or a zero
+TSU_HD bool small_or_zero(double x) {
+    const uint32_t t = hi32(x) & 0x7fffffffu;
+    return (t - 0x0df00000u < 0x44f00000u - 0x0df00000u) | ((t | lo32(x)) == 0u);
+}
 // The significand of a divisor is not all ones, judged by its low word (a few
 // other divisors take the fallback too).
 TSU_HD bool recip_ok(double d) { return lo32(d) != 0xffffffffu; }

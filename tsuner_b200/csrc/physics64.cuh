@@ -230,12 +230,16 @@ __device__ __forceinline__ void velocity_near_front(double h, double qx, double 
     clamp_speed(u, v, ok);
 }
 
+// |x| < 2^100: what a face's differences are made of must be (see limit)
+__device__ __forceinline__ bool limited(double x) { return (hi32(x) & 0x7fffffffu) < 0x46300000u; }
+
 // dry land: a state of zeros
 __device__ __forceinline__ bool empty(double h, double qx, double qy, double hc) {
     return ((hi32(h) | hi32(qx) | hi32(qy) | hi32(hc)) << 1 | lo32(h) | lo32(qx) | lo32(qy) | lo32(hc)) == 0u;
 }
 
-// Velocity and concentration of an unfiltered state (a cell, a ghost).
+// Velocity and concentration of an unfiltered state (a cell, a ghost).  FAST
+// takes only states whose depth, velocity and concentration are limited().
 template <bool FAST>
 __device__ __forceinline__ Face5 face_of(double h, double qx, double qy, double H, double hc, bool &ok) {
     Face5 f;
@@ -245,7 +249,8 @@ __device__ __forceinline__ Face5 face_of(double h, double qx, double qy, double 
         const Divisor<true> d(h + kEpsilon, ok);
         f.u = d.of(qx);
         f.v = d.of(qy);
-        f.c = d.of(hc, ok);
+        ok &= small_or_zero(hc);
+        f.c = d.of(hc);
         ok &= (wet_divisor(d.d) & calm(qx, f.u) & calm(qy, f.v)) | empty(h, qx, qy, hc);
     } else {
         velocity(h, qx, qy, f.u, f.v);
@@ -311,6 +316,8 @@ __device__ __forceinline__ Face5 filter_near_front(double h, double &qx, double 
 // avg, the van-Leer-type limiter (GPU/Reconstructor.cu:19-31): with a and b
 // of the same sign (a |b| + b |a|) / (|a| + |b|) is 2 a b / (a + b), every
 // operation rounding alike; of opposite sign its numerator is an exact zero.
+// Both only while nothing overflows: FAST needs a and b below 2^101 (larger
+// ones and infinities give a NaN by the general form, not a zero).
 template <bool FAST>
 __device__ __forceinline__ double limit(double a, double b, bool &ok) {
     if (!FAST) return limiter(a, b);
