@@ -21,8 +21,10 @@
 //  * quotient: q0 = a y, two corrections q <- q + y (a - d q).  The first
 //    leaves q faithful; the second, with a correctly rounded y and the exact
 //    residual of a faithful q, gives the correctly rounded quotient (same
-//    source, theorem 8's corollary).  Exponents in [-800, 800] keep every
-//    residual above the subnormal range.
+//    source, theorem 8's corollary).  Operands between 2^-800 and 2^800 whose
+//    quotient lies between 2^-1000 and 2^1000 keep every intermediate result
+//    and residual in the normal range; mid() tests the operands, and the bound
+//    on the quotient follows at each call site from what its divisor can be.
 //  * square root: the coupled iteration g -> sqrt(x), h -> 1/(2 sqrt(x)),
 //    r = 1/2 - g h, g <- g + g r, h <- h + h r (R. Goldschmidt, 1964), then
 //    g <- g + h (x - g^2).  After two steps g is within 0.51 ulp and h within
@@ -32,7 +34,8 @@
 //    last place), so the result is correctly rounded.
 // tests/ieee64_check.cpp checks both against the host's IEEE operations on
 // random operands, on the operands whose roots lie closest to a rounding
-// boundary, and over the seeds' error range.
+// boundary, and over the seeds' error range; tests/ieee64_device_check.cu the
+// device's own seeds (their error and the results) against its `/` and sqrt.
 #pragma once
 #include <cmath>
 #include <cstdint>
@@ -97,8 +100,9 @@ TSU_HD double recip_from(double d, double y) {
     e = fma64(-d, y, 1.0);
     return fma64(y, e, y);
 }
-// RN(a/d) from y = RN(1/d) and a first quotient q0 within a few thousand ulp;
-// mid_or_zero(a) (a zero numerator gives a zero, its sign not kept)
+// RN(a/d) from y = RN(1/d) and a first quotient q0 with |q0 d / a - 1| <= 2^-30
+// (the first correction leaves any such q0 faithful); mid_or_zero(a) (a zero
+// numerator gives a zero, its sign not kept)
 TSU_HD double quot_from(double a, double d, double y, double q0) {
     double r = fma64(-q0, d, a);
     const double q = fma64(r, y, q0);

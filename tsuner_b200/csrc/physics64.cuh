@@ -42,6 +42,9 @@ struct Phys64 {
     // without evaluating the Riemann solver (see edge_flux)
     int dry_skip;
     double inv_vs;  // RN(1 / k.vs)
+    // 1: the source terms always take the ordinary operators (Manning friction,
+    // or a divisor that the branch-free form could not take: see sources())
+    int plain_sources;
     // High word of a speed s such that two components below it leave the bed
     // at rest for certain: Opar (s^2 + s^2) < 0.99 OC (0: no such speed).
     unsigned still_hi;
@@ -150,14 +153,15 @@ struct Face5 {
 template <bool FAST>
 struct Divisor {
     double d, y;
-    // FAST: mid(d) is the caller's to know
+    // FAST: 2^-800 <= |d| < 2^800 and a quotient between 2^-1000 and 2^1000 are
+    // the caller's to know (each use below says from what)
     __device__ __forceinline__ Divisor(double d_, bool &ok) : d(d_), y(0.0) {
         if (FAST) {
             y = recip(d);
             ok &= recip_ok(d);
         }
     }
-    // numerator / d
+    // numerator / d; FAST tests 2^-800 <= |a| < 2^800 or a zero
     __device__ __forceinline__ double of(double a, bool &ok) const {
         if (!FAST) return ddiv(a, d);
         ok &= mid_or_zero(a);
@@ -317,7 +321,8 @@ __device__ __forceinline__ Face5 filter_near_front(double h, double &qx, double 
 // of the same sign (a |b| + b |a|) / (|a| + |b|) is 2 a b / (a + b), every
 // operation rounding alike; of opposite sign its numerator is an exact zero.
 // Both only while nothing overflows: FAST needs a and b below 2^101 (larger
-// ones and infinities give a NaN by the general form, not a zero).
+// ones and infinities give a NaN by the general form, not a zero), which also
+// bounds s, and 2 p / s from below, by 2^-900.
 template <bool FAST>
 __device__ __forceinline__ double limit(double a, double b, bool &ok) {
     if (!FAST) return limiter(a, b);
@@ -361,7 +366,7 @@ __device__ __forceinline__ double bed_flux_fast(const Phys64 &P, double h, doubl
     ok &= mid_or_zero(m2);
     const double m = root(m2), O = P.Opar * m * m;
     ok &= mid_or_zero(O);
-    const double K1 = Divisor<true>(m + kEpsilon, ok).of(17.0 * u, ok);
+    const double K1 = Divisor<true>(m + kEpsilon, ok).of(17.0 * u, ok);  // 2^-52 <= m + EPSILON < 2^5
     const double e = O - P.OC, f = root(O) - P.k.sqrt_OC;
     const bool live = (e > 0.0) & (f > 0.0) & (h > P.HQB) & (h > P.k.DS5);
     const double qb = K1 * P.Q * e * f;
@@ -406,7 +411,9 @@ __device__ __forceinline__ bool edge_flux(const Phys64 &P, const Face5 &a, const
 
     // Roe average + wave-speed bounds (GPU/SedFlux.cuh:181-199)
     const double hm = 0.5 * (h0 + h1);
-    if (FAST) ok &= mid_or_zero(h0) & mid_or_zero(h1);
+    // depths below 2^80 and velocities up to 10 m/s bound every divisor below:
+    // 2^-400 <= s0q + s1q < 2^41, 2^-52 < dS < 2^45
+    if (FAST) ok &= small_or_zero(h0) & small_or_zero(h1);
     const double s0q = root_of<FAST>(h0), s1q = root_of<FAST>(h1);
     const double ghm = kG * hm;
     double SL = a.u - root_of<FAST>(kG * h0), SR = b.u + root_of<FAST>(kG * h1);
@@ -582,7 +589,7 @@ __device__ __forceinline__ double cfl_dt(const Phys64 &P, double h, double qx, d
 // cells the smaller of dx / lx and dy / ly is dx over the larger speed (the
 // rounded quotient does not increase with the divisor).
 __device__ __forceinline__ bool cfl_dt_fast(const Phys64 &P, const Face5 &f, double &dt) {
-    bool ok = mid(f.h);
+    bool ok = mid(f.h);  // f.h of a wet filtered state: 2^-20 < h < 2^100, and so is lx, ly from below
     if (f.h == 0.0) {  // no speed: an infinite step
         dt = CUDART_INF;
         return true;

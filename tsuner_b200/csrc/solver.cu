@@ -177,6 +177,8 @@ static void fill_phys(TsuSolver *s) {
     P.inv_dy = 1.0 / p->dy;
     P.k = s->hconsts;
     P.inv_vs = 1.0 / s->hconsts.vs;
+    const double vs = s->hconsts.vs, eh = p->epsilon_h;
+    P.plain_sources = sw->manning || !(vs >= 0x1p-100 && vs < 0x1p100) || !(eh >= 0.0 && eh < 0x1p100);
     const double rest = std::sqrt(0.495 * p->OC / p->Opar);
     P.still_hi = (rest > 0.0 && rest < 1e30) ? hi32(rest) : 0u;
     P.npx = p->npx;

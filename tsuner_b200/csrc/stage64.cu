@@ -223,7 +223,8 @@ __device__ __noinline__ void put_edge_any(const Phys64 &P, Face5 a, Face5 b, int
 
 // Friction (GPU/Reconstructor.cu:33-55) on the momentum (k1, k2) and the
 // erosion/deposition rate phi (:57-88), from U^n = v0; one velocity
-// evaluation serves both.
+// evaluation serves both.  Divisors: h + EPSILON (2^-52 .. 2^100), h + eps_h
+// and vs (bounded by plain_sources), 1 + cf with cf < 2^132, 1 + 4.3e-7 Z^5.
 template <bool FAST, bool FRONT = false>
 __device__ __forceinline__ bool sources(const Phys64 &P, double dt, const double v0[5], double &k1, double &k2,
                                         double &phi) {
@@ -254,7 +255,9 @@ __device__ __forceinline__ bool sources(const Phys64 &P, double dt, const double
         k1 *= cm;
         k2 *= cm;
     } else {
-        const double cf = d0.of(dt * P.FR * modu, ok);
+        const double f = dt * P.FR * modu;
+        if (FAST) ok &= small_or_zero(f);
+        const double cf = d0.of(f);
         const Divisor<FAST> d1(1.0 + cf, ok);
         k1 = d1.of(k1, ok);
         k2 = d1.of(k2, ok);
@@ -289,7 +292,7 @@ __device__ __noinline__ Sources sources_any(const Phys64 &P, double dt, State5 v
     Sources r;
     r.k1 = k1;
     r.k2 = k2;
-    if (FRONT && !P.manning && sources<true, true>(P, dt, v0, r.k1, r.k2, r.phi)) return r;
+    if (FRONT && !P.plain_sources && sources<true, true>(P, dt, v0, r.k1, r.k2, r.phi)) return r;
     r.k1 = k1;
     r.k2 = k2;
     sources<false>(P, dt, v0, r.k1, r.k2, r.phi);
@@ -805,7 +808,7 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
         }
         {  // friction and erosion/deposition from U^n
             double k1 = vk[1], k2 = vk[2], phi;
-            if (P.manning || !sources<true>(P, dt, v0, k1, k2, phi)) {
+            if (P.plain_sources || !sources<true>(P, dt, v0, k1, k2, phi)) {
                 State5 v;
                 v.h = v0[0];
                 v.qx = v0[1];
