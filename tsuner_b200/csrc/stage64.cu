@@ -188,10 +188,11 @@ __device__ __forceinline__ bool make_faces(const double *sV, const double *sUC, 
     if (qminus) *qminus = (step != 1) ? m.qx : m.qy;
     return ok;
 }
-// FRONT: the near_front form first.  It pays on the small grids' tile, where one
-// face by the ordinary operators sets the time of the stage (48 x 36 cells with
-// a coast: 23.0 -> 19.7 us per step); the large tile's warps hide it, and its
-// registers cost them 2 %.
+// FRONT: the near_front form first (not for a wide tile).  It pays on the small
+// grids' tile, where one face by the ordinary operators sets the time of the
+// stage (48 x 36 cells with a coast: 23.0 -> 19.7 us per step), and on a tile
+// full of such faces (1021 x 773, every cell at 8.5 m/s: 400 -> 338); the large
+// tile's warps hide a few of them, and there it cost 2 %.
 template <int PS, bool FRONT>
 __device__ __noinline__ void make_faces_any(const double *sV, const double *sUC, int c, int step, double *dst,
                                             int fstride, int side, double *deta_out, double *qplus, double *qminus,
@@ -322,7 +323,10 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
     double *smem = smem_align<128>(smem_raw);
     __shared__ uint64_t sBar;     // the tile's TMA load
     __shared__ uint64_t sBarOwn;  // OWN == 2: the owned cells' U^n and extrema
-    __shared__ int sWide;         // the tile or its halo holds a cell that is not limited()
+    // cells of the tile and its halo that need the general form, and kWide for
+    // each that is not limited()
+    __shared__ int sOdd;
+    constexpr int kWide = 1 << 16;
     const Phys64 &P = A.phys;
     double *sV = smem;                  // [5][LY][LX]
     double *sUC = smem + T::kSV;        // [3][LY][LX]  (ux, uy, c)
@@ -345,7 +349,7 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
         mbar_init(&sBar, 1);
         if (OWN == 2 && !FIRST) mbar_init(&sBarOwn, 1);
         mbar_init_fence();
-        sWide = 0;
+        sOdd = 0;
     }
     prior_grids_done();
     next_grid_may_start();
@@ -460,19 +464,27 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
     }
 
     // ---- phase 2: per-cell velocity and concentration
+    int odd = 0;
     for (int idx = tid; idx < PS; idx += NT) {
         const double h = sV[idx], qx = sV[PS + idx], qy = sV[2 * PS + idx], hc = sV[4 * PS + idx];
         bool ok = true;
         Face5 f = face_of<true>(h, qx, qy, 0.0, hc, ok);
         if (!ok) {
             f = face_of<false>(h, qx, qy, 0.0, hc, ok);
-            if (!(limited(h) & limited(f.u) & limited(f.v) & limited(f.c))) sWide = 1;
+            odd += (limited(h) & limited(f.u) & limited(f.v) & limited(f.c)) ? 1 : kWide;
         }
         sUC[idx] = f.u;
         sUC[PS + idx] = f.v;
         sUC[2 * PS + idx] = f.c;
     }
+    if (odd) atomicAdd(&sOdd, odd);
     __syncthreads();
+    // A tile most of whose cells the branch-free form of the faces refuses
+    // (films, speeds from 7 m/s) does not try it first.  1021 x 773, every cell
+    // at 8.5 m/s: 459 -> 338 us per step, films of 3e-7 m: 380 -> 290; the same
+    // test for the sources and the update gave 4 % more there, but cost every
+    // other grid 0.4 %.
+    constexpr int kMost = PS / 2;
 
     // Periodic grids with an expired boundary series mirror the discharge of the
     // seam's low-side face into its high-side face (phase 4).  The faces do not
@@ -544,8 +556,8 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
     constexpr int RPW = 32 / TX, WX = TY / RPW, WY = (FYH + RPW - 1) / RPW, WF = (2 * TY + 31) / 32;
     static_assert(32 % TX == 0 && TY % RPW == 0, "tile rows per warp");
     const int warp = tid >> 5, lr = (tid & 31) / TX, lc = (tid & 31) % TX;
-    // The loop comes twice, with and without what only seams and wide tiles
-    // need: 4096^2 4195 us per step, 4226 with that in one loop.
+    // The loop comes twice, with and without what only these tiles need: 4096^2
+    // 4195 us per step, 4226 with that in one loop.
     auto faces = [&](const bool G) __attribute__((always_inline)) {
         for (int item = warp; item < ((RK0 && ORDER == 2) ? 0 : WX + WY + WF); item += NT / 32) {
             const bool xi = item < WX || item >= WX + WY;
@@ -591,9 +603,12 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
                     if (G && qminus) *qminus = 0.0;
                 } else {
                     double *deta = (didx >= 0) ? sDeta + didx : nullptr;
-                    if (G || !make_faces<PS, true>(sV, sUC, c, step, dst, fstride, side, deta))
-                        make_faces_any<PS, T::kSmall>(sV, sUC, c, step, dst, fstride, side, deta, qplus, qminus,
-                                                      sWide != 0);
+                    if (G)
+                        make_faces_any<PS, true>(sV, sUC, c, step, dst, fstride, side, deta, qplus, qminus,
+                                                 sOdd >= kWide);
+                    else if (!make_faces<PS, true>(sV, sUC, c, step, dst, fstride, side, deta))
+                        make_faces_any<PS, T::kSmall>(sV, sUC, c, step, dst, fstride, side, deta, nullptr, nullptr,
+                                                      false);
                 }
             } else {  // first order: faces are the cell values (GPU/Reconstructor.cu:99-107)
                 Face5 f;
@@ -610,7 +625,7 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
             }
         }
     };
-    const bool general = seam_q || sWide != 0;  // no branch-free form of this tile's faces
+    const bool general = seam_q || sOdd > kMost;  // no branch-free form of this tile's faces
     if (general) faces(true);
     else faces(false);
     __syncthreads();
