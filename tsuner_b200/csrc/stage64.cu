@@ -1060,9 +1060,22 @@ EncodeTiledFn tensor_map_encoder() {
 
 namespace {
 
-// At most one wave of 32 x 8 tiles (two CTAs on each of 148 SMs): 16 x 4 tiles
-// instead.  48 x 36 cells, 64 steps: 32 x 8 tiles 1017 us, 16 x 4 615 us.
-constexpr long long kSmallTiles = 296;
+// Grids of up to one wave of 16 x 4 tiles (three CTAs on each of 148 SMs) use
+// those: a tile is then one round of its warps, and more SMs have work.  Beyond
+// it they need a second wave, with 1.5 times the halo cells per owned one, where
+// 32 x 8 tiles need one.  On narrow grids, where most 32 x 8 tiles lie at a
+// boundary and wait for their few faces of the general form, the second wave
+// costs no more until it is two thirds full.  us per step, 16 x 4 against
+// 32 x 8, still water entered by a wave / moving water with humps:
+//   48 x 36 (27 tiles of 16 x 4)  18.2 / 21.0  26.8 / 31.4
+//   384 x 72 (432)                22.7 / 20.7  25.4 / 27.5
+//   768 x 44 (528)                34.7 / 27.0  28.9 / 23.5
+//   256 x 248 (992)               41.5 / 39.3  32.5 / 36.0
+//   128 x 224 (448)               28.5 / 26.9  28.9 / 31.9
+//   96 x 440 (660)                34.0 / 31.5  34.4 / 39.6
+//   96 x 592 (888)                40.6 / 36.8  33.8 / 38.6
+constexpr long long kSmallTiles = 444, kNarrowTiles = 740;
+constexpr int kNarrow = 256;  // columns; up to here the two are even between the limits
 
 struct Variant {
     int tx, ty, nthr, own;
@@ -1093,6 +1106,7 @@ const Variant &variant(int npx, int npy) {
     static const bool fixed = std::getenv("TSU_TILE64") != nullptr;
     static const Variant v = [] {
         const char *e = std::getenv("TSU_TILE64");
+        if (e && !std::strcmp(e, "32x8")) return make_variant<32, 8, 2, 320, 2>();  // the default, on every grid
         if (e && !std::strcmp(e, "16x16")) return make_variant<16, 16, 2>();
         if (e && !std::strcmp(e, "16x4")) return make_variant<16, 4, 3, 192, 2>();
         if (e && !std::strcmp(e, "32x8t256")) return make_variant<32, 8, 2, 256>();
@@ -1104,11 +1118,10 @@ const Variant &variant(int npx, int npy) {
         return make_variant<32, 8, 2, 320, 2>();
     }();
     // Small grids: 16 x 4 tiles of 192 threads.  Every phase of a tile is then
-    // one round of its six warps (the 32 x 8 tile needs two of its ten), and
-    // four times as many SMs have work.
+    // one round of its six warps (the 32 x 8 tile needs two of its ten).
     static const Variant small = make_variant<16, 4, 3, 192, 2>();
-    const long long tiles = (long long)((npx + 31) / 32) * ((npy + 7) / 8);
-    return (!fixed && tiles <= kSmallTiles) ? small : v;
+    const long long tiles = (long long)((npx + 15) / 16) * ((npy + 3) / 4);
+    return (!fixed && tiles <= (npx <= kNarrow ? kNarrowTiles : kSmallTiles)) ? small : v;
 }
 
 }  // namespace
