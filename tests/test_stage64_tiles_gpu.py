@@ -1,8 +1,13 @@
-"""GPU: the rule that picks one of the FP64 form's two tiles picks the faster one."""
+"""GPU: the FP64 form's two tiles.  The tests of the switches, boundary series,
+seams, slabs and mixed states run once with each tile forced on every grid (the
+size rule alone would leave most of them to the small tile), every kernel
+variant gives the same values on a grid of several tiles of each shape, and the
+rule that picks a tile picks the faster one."""
 import os
 import subprocess
 import sys
 
+import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -17,6 +22,42 @@ def run(args, tile, timeout=600):
     r = subprocess.run([sys.executable] + args, env=env, capture_output=True, text=True, timeout=timeout, cwd=ROOT)
     assert r.returncode == 0, (r.stdout + r.stderr)[-3000:]
     return r.stdout
+
+
+@pytest.mark.parametrize("tile", ["32x8", "16x4"])
+@pytest.mark.parametrize("tests,names", [
+    ("tests/test_parity_gpu.py", "vs_oracle or working_state or run_until or chunk"),
+    ("tests/test_stage64_paths_gpu.py", ""),
+    ("tests/test_slabs_gpu.py", ""),
+    ("tests/test_resume_gpu.py", "")])
+def test_small_grids_with_each_tile(tile, tests, names):
+    out = run(["-m", "pytest", "-q", "-x", "-m", "gpu", "-k", names, "-p", "no:cacheprovider", tests], tile)
+    assert " passed" in out and "skipped" not in out.splitlines()[-1], out[-500:]
+
+
+VALUES = """
+import sys, numpy as np
+import tsuner_b200 as T
+from tsuner_b200 import workloads as W
+w = W.nwave_shelf(%d, %d, 10.0, slr=0.5, amp=2.0, period=200.0, t_series=200.0)
+s = T.solver_for(w)
+s.step(20)
+hm, bm, em = s.extrema()
+np.savez(sys.argv[1], V=s.state(), hmax=hm, bmin=bm, eta_max=em, t=np.array(s.time()))
+s.close()
+"""
+
+
+@pytest.mark.parametrize("nx,ny", [(300, 200), (517, 203)])  # by rule 32 x 8; the second not a multiple of any tile
+def test_every_variant_gives_the_same_values(nx, ny, tmp_path):
+    out = {}
+    for tile in (None, "32x8", "16x4", "16x16", "32x8t256", "32x8t320reg", "32x8t320late"):
+        path = str(tmp_path / ("%s.npz" % tile))
+        run(["-c", VALUES % (nx, ny), path], tile)
+        out[tile] = np.load(path)
+    for tile, r in out.items():
+        for k in ("V", "hmax", "bmin", "eta_max", "t"):
+            assert np.array_equal(out[None][k], r[k]), (tile, k)
 
 
 TIME = """
