@@ -34,27 +34,70 @@ def test_run_until_enqueues_no_more_steps_than_dt_needs(precision):
         s.close()
 
 
-def test_finished_members_skip_their_tiles():
-    """A finished member is left before anything of its tiles is loaded.  Of a
-    live step it keeps the launches and two dependent reads per tile: well
-    below a quarter (24 members of 128^2 .. 1024^2: 158 of 750 us; loading the
-    tiles first takes 278)."""
-    ws = W.ensemble(nmembers=16, lo=256, hi=768, seed=5, t_series=200.0)
+def members(dxs, n=256):
+    """One hump per member; the coarser the grid, the larger its steps."""
+    ws = []
+    for k, dx in enumerate(dxs):
+        w = W.hump(n, n, dx, sigma=20.0 * dx, seed=k)
+        w.sw.precision = 1
+        ws.append(w)
+    return ws
+
+
+def ensemble(ws):
     e = T.Ensemble([w.p for w in ws], [w.sw for w in ws])
+    e.load(ws)
+    e.reset()
+    return e
+
+
+def test_finished_members_leave_the_tile_list():
+    """Steps of tsu_ens_run_until cost what the members that have not reached
+    the end time cost: nothing when all have (the steps still count), and as
+    much as an ensemble of the others when some have."""
+    coarse, fine = [80.0] * 6, [10.0] * 2
+    e, alone = ensemble(members(coarse + fine)), ensemble(members(fine))
     try:
-        e.load(ws)
-        e.reset()
-        e.step(32)
-        live, past = [], []
-        for _ in range(5):
-            e.step(32)
-            live.append(e.last_ms() / 32)
-            e.run_until(0.0, 64)
-            past.append(e.last_ms() / 64)
-        assert min(past) < 0.25 * min(live), (past, live)
+        t_end = 64 * e.members[0].time()[1]  # the coarse ones end after about 64 steps, the fine ones after 500
+        e.run_until(t_end, 128)
+        assert all(m.time()[0] >= t_end for m in e.members[:6])
+        assert all(m.time()[0] < 0.5 * t_end for m in e.members[6:])
         before = [m.state() for m in e.members]
-        e.run_until(0.0, 64)
-        for V, m in zip(before, e.members):
-            assert np.array_equal(V, m.state())
+        both, one = [], []
+        for _ in range(5):
+            assert e.run_until(t_end, 16) == 16
+            both.append(e.last_ms())
+            alone.step(16)
+            one.append(alone.last_ms())
+        assert min(both) < 1.3 * min(one), (both, one)
+        for k, m in enumerate(e.members):
+            assert np.array_equal(before[k], m.state()) == (k < 6)
+        t = [m.time() for m in e.members]
+        assert e.run_until(0.0, 100) == 64 and e.last_launches() == 0  # all have passed 0
+        assert [m.time() for m in e.members] == t
+    finally:
+        e.close()
+        alone.close()
+
+
+@pytest.mark.parametrize("config", [None, (0, 0, 0), (8, 1, 0)])  # default, static stride, dynamic
+def test_members_that_end_at_different_times_equal_members_alone(config):
+    ws = members([10.0, 45.0, 20.0, 80.0, 30.0], n=96)
+    e = ensemble(ws)
+    try:
+        if config:
+            e.set_config(*config)
+        t_end = 150 * e.members[3].time()[1]
+        n = e.run_until(t_end)
+        assert n % 64 == 0
+        for w, m in zip(ws, e.members):
+            s = T.solver_for(w)
+            try:
+                s.run_until(t_end)
+                assert s.time() == m.time() and np.array_equal(s.state(), m.state())
+            finally:
+                s.close()
+        e.step(1)  # the open end time and the whole list are back
+        assert all(m.time()[0] > t_end for m in e.members)
     finally:
         e.close()

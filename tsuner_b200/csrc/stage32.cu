@@ -744,14 +744,8 @@ __global__ void __launch_bounds__(TX *TY, MINB) ens32_kernel(EnsArgs E, Phys32 c
         P.npy = sG.phys.npy;
         P.wbc = sG.phys.wbc;
         P.read_files = sG.phys.read_files;
-        // Members end at different times under tsu_ens_run_until: a finished
-        // one is left before anything of its tile is loaded.  Looking first puts
-        // the read of the scalars in front of the loads' latency (1 % of a live
-        // step), so steps without an end time do not.  A step of 24 finished
-        // members of 128^2 .. 1024^2: 278 -> 158 us, a live one 750.
-        if (!E.until || load_written(sG.scal + SC_T) < load_written(sG.scal + SC_TEND))
-            stage32_tile<TX, TY, ORDER, FIRST, LAST>(sG, P, E.tmas ? E.tmas + m : nullptr, lt % ntx, lt / ntx, lt,
-                                                     E.members[m].ntiles, smem32);
+        stage32_tile<TX, TY, ORDER, FIRST, LAST>(sG, P, E.tmas ? E.tmas + m : nullptr, lt % ntx, lt / ntx, lt,
+                                                 E.members[m].ntiles, smem32);
         __syncthreads();
         if (E.dynamic) {
             if (threadIdx.x == 0) sTile = atomicAdd(E.work, 1u);

@@ -50,7 +50,6 @@ struct EnsArgs {
     // per member: TMA descriptors for the current tile shape, in device
     // memory (written before the launch), or null
     const Tma32 *tmas;
-    int until;  // an end time is set: a member that has reached it is left before anything of its tiles is loaded
 };
 
 size_t stage32_smem_bytes();
