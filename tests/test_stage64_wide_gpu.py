@@ -55,7 +55,10 @@ def odd_state(kind, nx, ny, seed=3):
     w = W.hump(nx, ny, 10.0, sigma=0.2 * nx * 10.0)
     w.V[3] = r.uniform(0.5, 3.0, (ny, nx))
     w.V[0] = w.V[3] + r.uniform(-0.2, 0.2, (ny, nx))
-    speed = {"calm": 0.5, "fast": 8.5, "clamped": 14.0, "film": 0.0}[kind] * r.uniform(0.95, 1.05, (ny, nx))
+    speed = {"calm": 0.5, "fast": 8.5, "clamped": 14.0, "film": 0.0, "scattered": 0.5}[kind]
+    speed = speed * r.uniform(0.95, 1.05, (ny, nx))
+    if kind == "scattered":
+        speed = np.where(r.uniform(size=(ny, nx)) < 0.05, 8.5, speed)
     if kind == "film":
         w.V[0] = 10.0 ** r.uniform(-7.0, -6.3, (ny, nx))
         speed = speed + 0.1
@@ -68,7 +71,7 @@ def odd_state(kind, nx, ny, seed=3):
 
 
 @pytest.mark.parametrize("nx,ny", [(48, 40), (640, 200), (641, 199)])
-@pytest.mark.parametrize("kind", ["fast", "clamped", "film"])
+@pytest.mark.parametrize("kind", ["fast", "clamped", "film", "scattered"])
 @pytest.mark.parametrize("wbc,order", [(1, 2), (2, 2), (0, 1)])
 def test_odd_tiles_equal_the_oracle(nx, ny, kind, wbc, order):
     w = odd_state(kind, nx, ny)

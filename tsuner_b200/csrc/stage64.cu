@@ -483,7 +483,9 @@ __global__ void __launch_bounds__(NTHR, MINB) stage64_kernel(const __grid_consta
     // (films, speeds from 7 m/s) does not try it first.  1021 x 773, every cell
     // at 8.5 m/s: 459 -> 338 us per step, films of 3e-7 m: 380 -> 290; the same
     // test for the sources and the update gave 4 % more there, but cost every
-    // other grid 0.4 %.
+    // other grid 0.4 %.  Fast cells one by one among calm ones (10 % of them: 477
+    // us) would gain from a lower line, 416 at PS / 32 and 379 at PS / 128, but
+    // the coast's tiles do not: 4096^2 8.87 -> 8.91 ms for two steps.
     constexpr int kMost = PS / 2;
 
     // Periodic grids with an expired boundary series mirror the discharge of the
