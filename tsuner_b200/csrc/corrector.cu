@@ -549,7 +549,7 @@ __host__ __device__ inline TileGeom tile_geom(int nimg, int H, int W) {
 
 // Weight (and bias) gradient partials of this CTA's tiles, written to its row
 // of `part` ([gridDim.x][kWgPart]: dW[cout][288], then the 4 warps' bias sums
-// [4][32]); wgrad_reduce_kernel adds the rows to dW and db in a fixed order, so
+// [4][32], then for each of them whether one is not finite); wgrad_reduce_kernel adds the rows to dW and db in a fixed order, so
 // the gradient does not depend on which CTA finishes first.
 //   warp 0: tile k (8 x 16 pixels) of X with one row of halo above and below,
 //     and of dZ with one column left and right, into a ring of kWgStages;
@@ -560,7 +560,8 @@ __host__ __device__ inline TileGeom tile_geom(int nimg, int H, int W) {
 //     X[p'] dZ[p' - dx] summed over p' is the tap's gradient: both operands
 //     are zero outside the image;
 //   warps 2-5: the bias gradient on the CUDA cores, a pixel per thread.
-constexpr int kWgPart = 32 * KROWS + 4 * 32;
+constexpr int kWgFlags = 32 * KROWS + 4 * 32;
+constexpr int kWgPart = kWgFlags + 32;  // rows of whole 128-byte lines
 __global__ void __launch_bounds__(kWgThreads, 1)
     conv3x3_wgrad_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmZ, int nimg,
                          int H, int W, float *__restrict__ part) {
@@ -751,6 +752,8 @@ __global__ void __launch_bounds__(kWgThreads, 1)
             if (lane == n) mine = v;
         }
         prow[32 * KROWS + (warp - 2) * 32 + lane] = mine;
+        const bool odd = __any_sync(0xffffffffu, !isfinite(mine));
+        if (lane == 0) prow[kWgFlags + warp - 2] = odd ? 1.f : 0.f;
     }
     fence_before();
     __syncthreads();
@@ -1074,14 +1077,40 @@ cudaError_t conv_launch(ConvArgs a, cudaStream_t st) {
     return cudaGetLastError();
 }
 
+// One tap's gradient of 32 input channels and output channel co by its
+// definition, sum over the pixels p of the images of dZ[p] X[p + off] with zeros
+// around X: what the tensor cores' products cannot give where an operand is not
+// finite, because they also multiply X by the zeros around dZ and leave out
+// those around X.  Lane: input channel; warp w of nw takes every nw-th pixel.
+__device__ __noinline__ double wgrad_direct(const bf16 *X, const bf16 *dZ, int nimg, int H, int W, int co, int tap,
+                                            int w, int nw) {
+    const int lane = threadIdx.x & 31, dy = tap / 3 - 1, dx = tap % 3 - 1;
+    const long long n = (long long)nimg * H * W;
+    double s = 0.0;
+    int k = 0;
+    for (long long p = w; p < n; p += nw) {
+        const long long row = p / W;
+        const int x = (int)(p - row * W) + dx, y = (int)(row % H) + dy;
+        const bool in = x >= 0 && x < W && y >= 0 && y < H;
+        const float z = __bfloat162float(dZ[p * C + co]);
+        const float v = in ? __bfloat162float(X[(p + (long long)dy * W + dx) * C + lane]) : 0.f;
+        s += (double)z * (double)v;
+        if ((++k & 255) == 0 && __all_sync(0xffffffffu, isnan(s))) break;  // nothing changes a NaN
+    }
+    return s;
+}
+
 // dW[k] (+)= sum over CTAs of part[b][k]; db[n] (+)= sum over CTAs and the 4
-// warps of the bias partials; added to what is there, or in its place.  A block owns 32 elements; each of its kRedWarps warps
-// takes every kRedWarps-th row (all loads in flight together: the kernel is a
-// latency, not a bandwidth), then the sums are added in order.
+// warps of the bias partials; added to what is there, or in its place.  A block
+// owns 32 elements; each of its kRedWarps warps takes every kRedWarps-th row
+// (all loads in flight together: the kernel is a latency, not a bandwidth), then
+// the sums are added in order.
 constexpr int kRedWarps = 16, kRedRows = 10;  // one pass covers 160 rows
 __global__ void __launch_bounds__(32 * kRedWarps)
-    wgrad_reduce_kernel(const float *part, int nctas, float *dW, float *db, bool add) {
+    wgrad_reduce_kernel(const float *part, int nctas, const bf16 *X, const bf16 *dZ, int nimg, int H, int W, float *dW,
+                        float *db, bool add) {
     __shared__ float sSum[kRedWarps][32];
+    __shared__ double sDirect[kRedWarps][32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int k = blockIdx.x * 32 + lane;
     const bool bias = k >= 32 * KROWS;  // the last block
@@ -1102,10 +1131,27 @@ __global__ void __launch_bounds__(32 * kRedWarps)
         for (int i = 0; i < kRedRows; i++) acc += v[i];
     }
     sSum[w][lane] = acc;
+    bool odd = false;  // a gradient or an element of X that is not finite
+    for (int b = threadIdx.x; b < nctas && !bias; b += 32 * kRedWarps) {
+        const float *f = part + (size_t)b * kWgPart + kWgFlags;
+        odd |= tsu::load_written(f) + tsu::load_written(f + 1) + tsu::load_written(f + 2) + tsu::load_written(f + 3) != 0.f;
+    }
     __syncthreads();
     if (w == 0) {
 #pragma unroll
         for (int q = 1; q < kRedWarps; q++) acc += sSum[q][lane];
+        odd |= !bias && !isfinite(acc);
+    }
+    if (__syncthreads_or(odd)) {
+        sDirect[w][lane] = wgrad_direct(X, dZ, nimg, H, W, blockIdx.x / 9, blockIdx.x % 9, w, kRedWarps);
+        __syncthreads();
+        if (w == 0) {
+            double s = sDirect[0][lane];
+            for (int q = 1; q < kRedWarps; q++) s += sDirect[q][lane];
+            acc = (float)s;
+        }
+    }
+    if (w == 0) {
         if (!bias) dW[k] = add ? dW[k] + acc : acc;
         else if (db) db[lane] = add ? db[lane] + acc : acc;
     }
@@ -1174,7 +1220,8 @@ cudaError_t wgrad_launch(const bf16 *X, const bf16 *dZ, int nimg, int H, int W, 
     launch_after(conv3x3_wgrad_kernel, dim3(ctas), dim3(kWgThreads), kWgSmem, st, mx, mz, nimg, H, W, part);
     e = cudaGetLastError();
     if (e == cudaSuccess) {
-        launch_after(wgrad_reduce_kernel, dim3(KROWS + 1), dim3(32 * kRedWarps), 0, st, part, ctas, dW, db, add);
+        launch_after(wgrad_reduce_kernel, dim3(KROWS + 1), dim3(32 * kRedWarps), 0, st, part, ctas, X, dZ, nimg, H, W, dW,
+                     db, add);
         e = cudaGetLastError();
     }
     if (own) {
