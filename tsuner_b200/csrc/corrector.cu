@@ -1081,21 +1081,22 @@ cudaError_t conv_launch(ConvArgs a, cudaStream_t st) {
 // definition, sum over the pixels p of the images of dZ[p] X[p + off] with zeros
 // around X: what the tensor cores' products cannot give where an operand is not
 // finite, because they also multiply X by the zeros around dZ and leave out
-// those around X.  Lane: input channel; warp w of nw takes every nw-th pixel.
+// those around X.  Lane: input channel; warp w of nw takes every nw-th row.
 __device__ __noinline__ double wgrad_direct(const bf16 *X, const bf16 *dZ, int nimg, int H, int W, int co, int tap,
                                             int w, int nw) {
     const int lane = threadIdx.x & 31, dy = tap / 3 - 1, dx = tap % 3 - 1;
-    const long long n = (long long)nimg * H * W;
     double s = 0.0;
-    int k = 0;
-    for (long long p = w; p < n; p += nw) {
-        const long long row = p / W;
-        const int x = (int)(p - row * W) + dx, y = (int)(row % H) + dy;
-        const bool in = x >= 0 && x < W && y >= 0 && y < H;
-        const float z = __bfloat162float(dZ[p * C + co]);
-        const float v = in ? __bfloat162float(X[(p + (long long)dy * W + dx) * C + lane]) : 0.f;
-        s += (double)z * (double)v;
-        if ((++k & 255) == 0 && __all_sync(0xffffffffu, isnan(s))) break;  // nothing changes a NaN
+    for (int r = w; r < nimg * H; r += nw) {
+        const int y = r % H + dy;
+        const bool in = y >= 0 && y < H;
+        const bf16 *z = dZ + (long long)r * W * C + co;
+        const bf16 *v = X + ((long long)(r + dy) * W + dx) * C + lane;
+#pragma unroll 8
+        for (int x = 0; x < W; x++) {
+            const float a = (in && x + dx >= 0 && x + dx < W) ? __bfloat162float(v[(long long)x * C]) : 0.f;
+            s += (double)__bfloat162float(z[(long long)x * C]) * (double)a;
+        }
+        if (__all_sync(0xffffffffu, isnan(s))) break;  // nothing changes a NaN
     }
     return s;
 }
