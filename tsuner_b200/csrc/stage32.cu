@@ -139,7 +139,8 @@ __device__ __forceinline__ void recon32(const Phys32 &P, const float *s, int c, 
 // P: the grid's physical parameters (A.phys, or the ensemble's shared
 // parameters with this member's grid fields).
 // tm: TMA descriptors of the state buffers (single grid), or null (ensemble).
-template <int TX, int TY, int ORDER, bool FIRST, bool LAST>
+// AHEAD: see the loads of tiles without a TMA box.
+template <int TX, int TY, int ORDER, bool FIRST, bool LAST, bool AHEAD>
 __device__ __forceinline__ void stage32_tile(const Stage32Args &A, const Phys32 &P, const Tma32 *tm, int bx, int by,
                                              unsigned blin, unsigned nb, float *smem_raw) {
     using T = T32<TX, TY>;
@@ -205,18 +206,37 @@ __device__ __forceinline__ void stage32_tile(const Stage32Args &A, const Phys32 
         tma_load_2d(sM, &tm->m, x0 - MHX, y0 - 2, &sBar);
     }
     if (!use_tma) {
-        for (int k = tid; k < PSC; k += NT) {
-            const int ly = k / LXC, lxc = k - ly * LXC;
-            const int idx = ly * LX + lxc + (HX - 2);
-            int gx = x0 + lxc - 2, gy = y0 + ly - 2;
-            if (!inner) {
-                gx = wrap_clamp32(gx, npx, periodic);
-                gy = wrap_clamp32(gy, npy, periodic);
-            }
-            const long long g = (long long)gy * pitch + gx;
+        // AHEAD: all of a thread's cells requested before the first is stored, the
+        // loads' order being kept (48 x 36 cells: 17.2 -> 16.8 us per step, 8192^2
+        // 6.80 -> 6.76 ms; the ensemble's kernels lose 2 % by the registers).
+        constexpr int IT = AHEAD ? (PSC + NT - 1) / NT : 1;
+        float v[IT][5];
+        unsigned char m[IT];
+        for (int k0 = tid; k0 < PSC; k0 += IT * NT) {
 #pragma unroll
-            for (int f = 0; f < 5; f++) sV[f * PS + idx] = load_written(Vin + f * plane + g);
-            sM[ly * MLX + lxc + (MHX - 2)] = __ldg(A.mask + g);
+            for (int q = 0; q < IT; q++) {
+                const int k = k0 + q * NT;
+                if (k >= PSC) continue;
+                const int ly = k / LXC, lxc = k - ly * LXC;
+                int gx = x0 + lxc - 2, gy = y0 + ly - 2;
+                if (!inner) {
+                    gx = wrap_clamp32(gx, npx, periodic);
+                    gy = wrap_clamp32(gy, npy, periodic);
+                }
+                const long long g = (long long)gy * pitch + gx;
+#pragma unroll
+                for (int f = 0; f < 5; f++) v[q][f] = load_written(Vin + f * plane + g);
+                m[q] = __ldg(A.mask + g);
+            }
+#pragma unroll
+            for (int q = 0; q < IT; q++) {
+                const int k = k0 + q * NT;
+                if (k >= PSC) continue;
+                const int ly = k / LXC, lxc = k - ly * LXC;
+#pragma unroll
+                for (int f = 0; f < 5; f++) sV[f * PS + ly * LX + lxc + (HX - 2)] = v[q][f];
+                sM[ly * MLX + lxc + (MHX - 2)] = m[q];
+            }
         }
     }
     const int tx = tid % TX, ty = tid / TX;
@@ -697,7 +717,7 @@ __global__ void __launch_bounds__(TX *TY, MINB)
     extern __shared__ __align__(16) float smem32[];
     prior_grids_done();
     next_grid_may_start();
-    stage32_tile<TX, TY, ORDER, FIRST, LAST>(A, A.phys, &M, blockIdx.x, blockIdx.y,
+    stage32_tile<TX, TY, ORDER, FIRST, LAST, true>(A, A.phys, &M, blockIdx.x, blockIdx.y,
                                              blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y, smem32);
 }
 
@@ -744,7 +764,7 @@ __global__ void __launch_bounds__(TX *TY, MINB) ens32_kernel(EnsArgs E, Phys32 c
         P.npy = sG.phys.npy;
         P.wbc = sG.phys.wbc;
         P.read_files = sG.phys.read_files;
-        stage32_tile<TX, TY, ORDER, FIRST, LAST>(sG, P, E.tmas ? E.tmas + m : nullptr, lt % ntx, lt / ntx, lt,
+        stage32_tile<TX, TY, ORDER, FIRST, LAST, false>(sG, P, E.tmas ? E.tmas + m : nullptr, lt % ntx, lt / ntx, lt,
                                                  E.members[m].ntiles, smem32);
         __syncthreads();
         if (E.dynamic) {
