@@ -29,11 +29,11 @@ static int both_convolutions(int device) {
 // shared-memory attribute and SM count
 static int two_devices() {
     if (both_convolutions(0) || both_convolutions(1) || both_convolutions(0)) return 1;
-    // 4000 rows in one image, 8 columns: the launch fills the device it is for
+    // 4000 rows of nine column groups: the launch fills the device it is for
     for (int d = 0; d < 2; d++) {
         cudaSetDevice(d);
         fake::launches.clear();
-        EXPECT(tsu_corr_conv3x3(X, 1, 4000, 8, Wk, nullptr, 0, nullptr, Y, nullptr, nullptr) == TSU_OK);
+        EXPECT(tsu_corr_conv3x3(X, 1, 4000, 72, Wk, nullptr, 0, nullptr, Y, nullptr, nullptr) == TSU_OK);
         EXPECT(fake::launches.size() == 1 && fake::launches[0].grid == 2u * fake::sms[d]);
         fake::launches.clear();
         EXPECT(tsu_corr_conv3x3_wgrad(X, Z, 1, 16 * 300, 8, dW, db, nullptr) == TSU_OK);

@@ -37,6 +37,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
@@ -593,7 +594,7 @@ __host__ __device__ inline TileGeom tile_geom(int nimg, int H, int W) {
 
 // Weight (and bias) gradient partials of this CTA's tiles, written to its row
 // of `part` ([gridDim.x][kWgPart]: dW[cout][288], then the 4 warps' bias sums
-// [4][32], then for each of them whether one is not finite); wgrad_reduce_kernel adds the rows to dW and db in a fixed order, so
+// [4][32], then whether one of them is not finite); wgrad_reduce_kernel adds the rows to dW and db in a fixed order, so
 // the gradient does not depend on which CTA finishes first.
 //   warp 0: tile k (8 x 16 pixels) of X with one row of halo above and below,
 //     and of dZ with one column left and right, into a ring of kWgStages;
@@ -618,7 +619,7 @@ __global__ void __launch_bounds__(kWgThreads, 1)
     uint64_t *fin = acce + 2;            // all MMAs done
     uint32_t *tslot = reinterpret_cast<uint32_t *>(fin + 1);
     int *sCount = reinterpret_cast<int *>(tslot + 1);  // [0] stages issued, [1] stages waited for by the MMA warp
-    int *sFail = sCount + 2;
+    int *sFail = sCount + 2, *sOdd = sCount + 3;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const TileGeom G = tile_geom(nimg, H, W);
     const int ntile = (int)blockIdx.x < G.total ? (G.total - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
@@ -634,7 +635,7 @@ __global__ void __launch_bounds__(kWgThreads, 1)
         }
         mbar_init(fin, 1);
         sCount[0] = sCount[1] = 0;
-        *sFail = 0;
+        *sFail = *sOdd = 0;
         mbar_init_fence();
     }
     // TMEM is taken only now: a grid that holds some while it waits could starve
@@ -796,12 +797,12 @@ __global__ void __launch_bounds__(kWgThreads, 1)
             if (lane == n) mine = v;
         }
         prow[32 * KROWS + (warp - 2) * 32 + lane] = mine;
-        const bool odd = __any_sync(0xffffffffu, !isfinite(mine));
-        if (lane == 0) prow[kWgFlags + warp - 2] = odd ? 1.f : 0.f;
+        if (!isfinite(mine)) atomicExch(sOdd, 1);
     }
     fence_before();
     __syncthreads();
     fence_after();
+    if (tid == 0) prow[kWgFlags] = *sOdd ? 1.f : 0.f;
     if (warp == 1) tmem_dealloc(tmem, 256);
 }
 
@@ -1068,9 +1069,9 @@ cudaError_t make_map(CUtensorMap *m, const void *base, int nimg, int H, int W, i
 // attribute, the SM count, the pool of the calls that bring no scratch.
 constexpr int kMaxDevices = 64;
 struct DeviceState {
-    bool ready = false;
-    int sms = 0;
-    cudaMemPool_t pool = nullptr;
+    std::atomic<bool> ready{false};
+    std::atomic<int> sms{0};
+    cudaMemPool_t pool = nullptr;  // under g_dev_mu
 };
 std::mutex g_dev_mu;
 DeviceState g_dev[kMaxDevices];
@@ -1083,25 +1084,24 @@ DeviceState *device_state() {
 
 // the kernels' shared memory on the current device
 cudaError_t prepare() {
-    std::lock_guard<std::mutex> g(g_dev_mu);
     DeviceState *d = device_state();
-    if (d && d->ready) return cudaSuccess;
+    if (d && d->ready.load(std::memory_order_acquire)) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(conv3x3_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(conv3x3_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgSmem);
-    if (e == cudaSuccess && d) d->ready = true;
+    if (e == cudaSuccess && d) d->ready.store(true, std::memory_order_release);
     return e;
 }
 
 // SMs of the current device
 int num_sms() {
-    std::lock_guard<std::mutex> g(g_dev_mu);
     DeviceState *d = device_state();
-    if (d && d->sms) return d->sms;
+    if (d)
+        if (const int k = d->sms.load(std::memory_order_relaxed)) return k;
     int dev = 0, n = 0;
     cudaGetDevice(&dev);
     if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) n = 148;
-    if (d) d->sms = n;
+    if (d) d->sms.store(n, std::memory_order_relaxed);
     return n;
 }
 
@@ -1163,6 +1163,9 @@ __global__ void __launch_bounds__(32 * kRedWarps)
     float acc = 0.f;
     prior_grids_done();
     next_grid_may_start();
+    float flags = 0.f;  // first, so that they arrive with the sums
+    for (int b = threadIdx.x; b < nctas && !bias; b += 32 * kRedWarps)
+        flags += tsu::load_written(part + (size_t)b * kWgPart + kWgFlags);
     for (int b0 = w; b0 < n; b0 += kRedWarps * kRedRows) {
         float v[kRedRows];
 #pragma unroll
@@ -1176,11 +1179,7 @@ __global__ void __launch_bounds__(32 * kRedWarps)
         for (int i = 0; i < kRedRows; i++) acc += v[i];
     }
     sSum[w][lane] = acc;
-    bool odd = false;  // a gradient or an element of X that is not finite
-    for (int b = threadIdx.x; b < nctas && !bias; b += 32 * kRedWarps) {
-        const float *f = part + (size_t)b * kWgPart + kWgFlags;
-        odd |= tsu::load_written(f) + tsu::load_written(f + 1) + tsu::load_written(f + 2) + tsu::load_written(f + 3) != 0.f;
-    }
+    bool odd = flags != 0.f;  // a gradient (below: or an element of X) that is not finite
     __syncthreads();
     if (w == 0) {
 #pragma unroll
