@@ -20,7 +20,7 @@
 // whose M = 128 rows are 16 groups of 8 pixels of one image row each and whose
 // N = 96 columns are the contributions of an input row to the three output
 // rows around it, 6 MMAs (3 column offsets x 2 channel halves, K = 16) per
-// input row.  8 x 528^2 pixels, BF16 with ReLU: 103 -> 65 us from HBM (the 285
+// input row.  8 x 528^2 pixels, BF16 with ReLU: 103 -> 64 us from HBM (the 285
 // MB it reads and writes take 44 us).
 //
 // Weight gradient (conv3x3_wgrad_kernel): dW[cout][tap][cin] =
